@@ -466,7 +466,11 @@ cudaError_t launchTiled(const DevSynthesis &d, const DevTiled &t, const int* h_t
   const int agrid = atomGrid(ae - ab, sm_count);
   const int nmol = mol_end - mol_begin;
   if (vale) {
-    const dim3 vgrid(nmol, 4);
+    // four blocks a molecule when there are many; a lone molecule's chunks of 32 terms spread
+    // over up to 32 blocks (one 2,500-atom chain: 23 us on 4 blocks, 10 on 32)
+    int vrows = 2 * sm_count / nmol;
+    vrows = vrows < 4 ? 4 : (vrows > 32 ? 32 : vrows);
+    const dim3 vgrid(nmol, vrows);
 #define SB_VALE(C)                                                                             \
     if (force && energy) kTiledValence<true, true, C><<<vgrid, 256, 0, stream>>>(d, t, mol_begin); \
     else if (force) kTiledValence<true, false, C><<<vgrid, 256, 0, stream>>>(d, t, mol_begin);   \
