@@ -8,7 +8,9 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <limits>
 #include <memory>
+#include <mutex>
 #include <set>
 #include <stdexcept>
 #include <string>
@@ -62,8 +64,10 @@ cudaError_t launchRestraints(const DevCharmm &c, int first, int count, bool forc
 cudaError_t launchSurfaceArea(const long long* xcrd, const long long* ycrd,
                               const long long* zcrd, double inv_gpos_scale,
                               const int* atom_start, const int* atom_count, int nsys,
-                              const double* radius, const double3* pts, int npts, double probe,
-                              double weight, int* cell, double* out, cudaStream_t stream);
+                              const int* map, int natom, const double* radius,
+                              const double3* pts, int npts, double stretch, double probe,
+                              double weight, double4* at, int* cell, int* shape, double* area,
+                              double* out, cudaStream_t stream);
 
 namespace {
 thread_local std::string g_last_error;
@@ -1531,25 +1535,41 @@ void Synthesis::surfaceArea(const double* points, int npts, double probe, double
     throw Error(SB_ERR_ARGUMENT, "surface area: points, a positive point count, a finite "
                 "non-negative probe and a finite weight are required");
   }
+  // the longest point bounds how far a sphere of points reaches; one that is not finite makes
+  // the bound infinite, which leaves no atom out
   std::vector<double3> pts(npts);
+  double longest = 0.0;
   for (int p = 0; p < npts; p++) {
     pts[p] = make_double3(points[3 * p], points[3 * p + 1], points[3 * p + 2]);
+    const double len = std::sqrt(pts[p].x * pts[p].x + pts[p].y * pts[p].y +
+                                 pts[p].z * pts[p].z);
+    longest = std::isfinite(len) ? std::max(longest, len) :
+                                   std::numeric_limits<double>::infinity();
   }
-  DeviceArray<double> radius, result;
-  DeviceArray<double3> d_pts;
-  DeviceArray<int> cell;
-  radius.allocate(h_sasa_radius.size());
-  d_pts.allocate(npts);
-  cell.allocate(h_sasa_radius.size());
-  result.allocate(nsys);
-  cudaCheck(cudaMemcpyAsync(radius.p, h_sasa_radius.data(), h_sasa_radius.size() * sizeof(double),
+  // the call holds the scratch until its results are back
+  std::lock_guard<std::mutex> lock(sasa_mutex);
+  if (d_sasa_at.p == nullptr) {
+    UploadArena arena;
+    arena.put(&d_sasa_radius, h_sasa_radius);
+    arena.zero(&d_sasa_at, h_sasa_radius.size());
+    arena.zero(&d_sasa_area, h_sasa_radius.size());
+    arena.zero(&d_sasa_cell, h_sasa_radius.size());
+    arena.zero(&d_sasa_shape, nsys);
+    arena.zero(&d_sasa_out, nsys);
+    arena.commit(&d_sasa_arena);
+  }
+  if (d_sasa_pts.n < pts.size()) {
+    d_sasa_pts.allocate(pts.size());
+  }
+  cudaCheck(cudaMemcpyAsync(d_sasa_pts.p, pts.data(), npts * sizeof(double3),
                             cudaMemcpyHostToDevice, stream), "surface area upload");
-  cudaCheck(cudaMemcpyAsync(d_pts.p, pts.data(), npts * sizeof(double3), cudaMemcpyHostToDevice,
-                            stream), "surface area upload");
   cudaCheck(launchSurfaceArea(d_xcrd.p, d_ycrd.p, d_zcrd.p, std::ldexp(1.0, -opt.gpos_bits),
-                              d_atom_start.p, d_atom_count.p, nsys, radius.p, d_pts.p, npts,
-                              probe, weight, cell.p, result.p, stream), "surface area launch");
-  cudaCheck(cudaMemcpyAsync(out, result.p, nsys * sizeof(double), cudaMemcpyDeviceToHost,
+                              d_atom_start.p, d_atom_count.p, nsys, d_unpadded_map.p,
+                              natom_total, d_sasa_radius.p, d_sasa_pts.p, npts,
+                              longest, probe, weight, d_sasa_at.p, d_sasa_cell.p,
+                              d_sasa_shape.p, d_sasa_area.p, d_sasa_out.p, stream),
+            "surface area launch");
+  cudaCheck(cudaMemcpyAsync(out, d_sasa_out.p, nsys * sizeof(double), cudaMemcpyDeviceToHost,
                             stream), "surface area download");
   cudaCheck(cudaStreamSynchronize(stream), "surface area");
 }

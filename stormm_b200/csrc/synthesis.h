@@ -13,6 +13,7 @@
 
 #include <functional>
 #include <memory>
+#include <mutex>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -318,6 +319,13 @@ public:
   int fused_tiles = 0;           // tiles of all molecules on the fused path
   DeviceArray<int> d_unpadded_map;
   DeviceArray<double> d_stage_xyz, d_stage_nrg;
+  // surface-area scratch, built by the first call and held by one call at a time
+  std::mutex sasa_mutex;
+  DeviceArray<unsigned char> d_sasa_arena;
+  DeviceArray<double> d_sasa_radius, d_sasa_area, d_sasa_out;
+  DeviceArray<double4> d_sasa_at;
+  DeviceArray<double3> d_sasa_pts;
+  DeviceArray<int> d_sasa_cell, d_sasa_shape;
   DeviceArray<int> d_tiled_systems, d_tile_prefix, d_atom_prefix;
   DeviceArray<long long> d_tiled_psi, d_tiled_de;
   DeviceArray<float> d_tiled_radius, d_tiled_sde;
