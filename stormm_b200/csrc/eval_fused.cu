@@ -17,17 +17,7 @@
 //   pass 3      radius chain-rule forces (nonbonded_potential.tpp:1022-1290)
 //   commit      forces into the int64 + int32-overflow arrays, energies into per-system slots
 //
-// Pair passes walk 32 x 32 tiles of a molecule's lower triangle, one tile per warp.  Lane l
-// holds atom i = I*32 + l in registers; j atoms rotate through the lanes (lane l meets atom
-// (l + k) mod 32 of block J at step k) and j-side accumulators travel with a shuffle per step.
-// Diagonal tiles take 16 steps, the last one on half the lanes, so every pair is visited once.
-// Forces, psi and dE/dR leave registers once per tile through integer shared-memory atomics,
-// so every sum is independent of scheduling and the results are bit-identical run to run.
-//
-// Shared memory per atom slot: pos_a = (x_hi, y_hi, z_hi, w1) and pos_b = (x_lo, y_lo, z_lo, w2)
-// feed the pair passes with two 16-byte loads per partner; w1 / w2 carry what the pass needs
-// (pass 1 and 3: s*rho and rho; pass 2: charge and effective radius).  prm holds the static
-// per-atom values, gbv the reciprocal effective radius and the chain-rule dE/dR.
+// The passes, their tile walks and the shared-memory layout are in unit_eval.cuh.
 #include "unit_eval.cuh"
 
 namespace sb {

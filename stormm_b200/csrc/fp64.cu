@@ -152,8 +152,41 @@ __device__ __forceinline__ double hctDerivative64(double r, double rho, double s
   return 0.0;
 }
 
+// Run one tile: p.pair(jslot, jl) for every pair of the tile (once each) and p.rotate() after
+// every step.  Lane l holds block I's atom l, block J's atoms and their accumulators rotate through
+// the lanes; a diagonal tile takes 16 steps, the last on half the lanes, where lanes l and l + 16
+// would meet the same pair.
+template <class P>
+__device__ __forceinline__ void walkTile64(P &p, const TileInfo &ti, int lane) {
+  if (!ti.diag) {
+#pragma unroll 2
+    for (int k = 0; k < kTile; k++) {
+      const int jl = (lane + k) & 31;
+      p.pair(ti.jbase + jl, jl);
+      p.rotate(lane);
+    }
+  }
+  else {
+#pragma unroll 1
+    for (int k = 1; k < 16; k++) {
+      const int jl = (lane + k) & 31;
+      p.pair(ti.jbase + jl, jl);
+      p.rotate(lane);
+    }
+    if (lane < 16) {
+      p.pair(ti.jbase + lane + 16, lane + 16);
+    }
+    p.rotate(lane);
+  }
+}
+
+// Lane that holds block J's atom jl's traveling accumulator once the walk is over
+__device__ __forceinline__ int traveledAtom(const TileInfo &ti, int lane) {
+  return (lane + (ti.diag ? 17 : 32)) & 31;
+}
+
 // ------------------------------------------------------------------------------------------------
-// Pair functors for walkTile (lane l holds block I's atom, block J's atoms rotate)
+// Pair functors for walkTile64
 // ------------------------------------------------------------------------------------------------
 // Pass 1 payload: w1 = s * rho, w2 = rho, code = neck index
 struct Radii64 {
@@ -410,7 +443,7 @@ kRadii64(const DevSynthesis d, const DevPrecise p, const DevTiled t, int tile_be
     const TileInfo ti = tiledTileInfo(d, sysid, g - t.tile_prefix[m], &I, &J);
     stageTile64<1>(d, p, t, v, sysid, I, J, ti.diag, lane);
     f.begin(lane);
-    walkTile(f, ti, lane);
+    walkTile64(f, ti, lane);
     const int base = d.atom_start[sysid];
     if (lane < ti.ni) {
       addFixed(&t.psi_acc[base + I * kTile + lane], f.psi_i * kAcc64Scale);
@@ -454,7 +487,7 @@ kPair64(const DevSynthesis d, const DevPrecise p, const DevTiled t, int tile_beg
       f.qc = quadraticCore64(f.cl.x);
     }
     f.begin(lane, mask);
-    walkTile(f, ti, lane);
+    walkTile64(f, ti, lane);
     const int base = d.atom_start[sysid];
     if (FORCE) {
       if (lane < ti.ni) {
@@ -508,7 +541,7 @@ kDeriv64(const DevSynthesis d, const DevPrecise p, const DevTiled t, int tile_be
     const TileInfo ti = tiledTileInfo(d, sysid, g - t.tile_prefix[m], &I, &J);
     stageTile64<3>(d, p, t, v, sysid, I, J, ti.diag, lane);
     f.begin(lane);
-    walkTile(f, ti, lane);
+    walkTile64(f, ti, lane);
     const int base = d.atom_start[sysid];
     if (lane < ti.ni) {
       const int gi = base + I * kTile + lane;

@@ -307,7 +307,7 @@ public:
   DeviceArray<long long> d_psi, d_sumdeijda;
   DeviceArray<int> d_psi_ovrf, d_sumdeijda_ovrf, d_status;
   DeviceArray<float> d_born_radii;
-  DeviceArray<float2> d_pair_deriv;
+  DeviceArray<float4> d_pair_deriv;
   std::vector<int> h_neck_idx;
   std::vector<float> h_neck_sep, h_neck_val;
   std::vector<double> h64_neck_sep, h64_neck_val;

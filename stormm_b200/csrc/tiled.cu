@@ -31,43 +31,23 @@ struct GlobalValence {
   const int* dchunk0;
   const int* sys;
   const int* slot0;
-  const float2* lj14tab;
-  int nt;
   __device__ GlobalValence(const DevSynthesis &d_in, const int* chunks, const int* sys_in,
-                           const int* slot0_in, const float2* lj14_in, int nt_in) :
+                           const int* slot0_in) :
       d(d_in), bchunk0(chunks), achunk0(chunks + 2), dchunk0(chunks + 4), sys(sys_in),
-      slot0(slot0_in), lj14tab(lj14_in), nt(nt_in) {}
+      slot0(slot0_in) {}
   __device__ __forceinline__ int chunkBegin() const {
     return (threadIdx.x >> 5) + blockIdx.y * (blockDim.x >> 5);
   }
   __device__ __forceinline__ int chunkStride() const { return (blockDim.x >> 5) * gridDim.y; }
-  __device__ __forceinline__ void hilo(int i, float4* a, float4* b) const {
-    splitCoordinate(static_cast<double>(d.xcrd[i]) * d.inv_gpos_scale, &a->x, &b->x);
-    splitCoordinate(static_cast<double>(d.ycrd[i]) * d.inv_gpos_scale, &a->y, &b->y);
-    splitCoordinate(static_cast<double>(d.zcrd[i]) * d.inv_gpos_scale, &a->z, &b->z);
-    a->w = 0.0f;
-    b->w = 0.0f;
+  __device__ __forceinline__ float3 part(int i, bool high) const {
+    float3 h, l;
+    splitCoordinate(static_cast<double>(d.xcrd[i]) * d.inv_gpos_scale, &h.x, &l.x);
+    splitCoordinate(static_cast<double>(d.ycrd[i]) * d.inv_gpos_scale, &h.y, &l.y);
+    splitCoordinate(static_cast<double>(d.zcrd[i]) * d.inv_gpos_scale, &h.z, &l.z);
+    return high ? h : l;
   }
-  __device__ __forceinline__ float4 pa(int i) const {
-    float4 a, b;
-    hilo(i, &a, &b);
-    return a;
-  }
-  __device__ __forceinline__ float4 pb(int i) const {
-    float4 a, b;
-    hilo(i, &a, &b);
-    return b;
-  }
-  __device__ __forceinline__ float4 prm(int i) const {
-    const int ty = d.lj_idx[i];
-    return make_float4(d.charge[i], __int_as_float((ty * nt) | (ty << 16)), d.rho[i], d.srho[i]);
-  }
-  __device__ __forceinline__ float3 delta(int a, int b) const {
-    float4 aa, ab, ba, bb;
-    hilo(a, &aa, &ab);
-    hilo(b, &ba, &bb);
-    return pairDelta(aa, ab, ba, bb);
-  }
+  __device__ __forceinline__ float3 hi(int i) const { return part(i, true); }
+  __device__ __forceinline__ float3 lo(int i) const { return part(i, false); }
   __device__ __forceinline__ void force(int i, float fx, float fy, float fz, float scale) const {
     atomicAdd(reinterpret_cast<unsigned long long*>(&d.xfrc[i]),
               static_cast<unsigned long long>(__float2ll_rn(fx * scale)));
@@ -81,9 +61,6 @@ struct GlobalValence {
     if ((threadIdx.x & 31) == 0 && v != 0) {
       atomicAdd(&d.energies[sys[k] * kNrgStride + slot], static_cast<unsigned long long>(v));
     }
-  }
-  __device__ __forceinline__ float2 lj14(int code_i, int code_l, int) const {
-    return lj14tab[(code_i & 0xffff) + (code_l >> 16)];
   }
   __device__ __forceinline__ double3 pos64(int i) const {
     return make_double3(static_cast<double>(d.xcrd[i]) * d.inv_gpos_scale,
@@ -132,8 +109,7 @@ kTiledValence(const DevSynthesis d, const DevTiled t, int mol_begin) {
     chunks[5] = (d.dihe_start[s + 1] - d.dihe_start[s] + 31) / 32;
   }
   __syncthreads();
-  const int s = sys[0];
-  const GlobalValence v(d, chunks, sys, slot0, d.ljab14 + d.lj_start[s], d.lj_ntypes[s]);
+  const GlobalValence v(d, chunks, sys, slot0);
   valenceTerms<FORCE, ENERGY, GlobalValence, CLASH>(d, v, 1);
 }
 
@@ -150,61 +126,56 @@ __device__ __forceinline__ void stageTile(const DevSynthesis &d, const DevTiled 
   for (int half = 0; half < (diag ? 1 : 2); half++) {
     const int a = (half == 0 ? I : J) * kTile + lane;
     const int slot = half * kTile + lane;
-    float4 pa, pb, prm;
-    float2 gbv = make_float2(1.0f, 0.0f);
+    float3 hi = make_float3(5000.0f + 16.0f * static_cast<float>(slot), 0.0f, 0.0f);
+    float3 lo = make_float3(0.0f, 0.0f, 0.0f);
+    float w1 = 0.0f, w2 = 1.0f, g = 1.0f, h = 0.0f;
     if (a < natom) {
       const int gi = base + a;
-      pa.w = 0.0f;
-      pb.w = 0.0f;
-      splitCoordinate(static_cast<double>(d.xcrd[gi]) * d.inv_gpos_scale, &pa.x, &pb.x);
-      splitCoordinate(static_cast<double>(d.ycrd[gi]) * d.inv_gpos_scale, &pa.y, &pb.y);
-      splitCoordinate(static_cast<double>(d.zcrd[gi]) * d.inv_gpos_scale, &pa.z, &pb.z);
-      const int ty = d.lj_idx[gi];
-      prm = make_float4(d.charge[gi], __int_as_float((ty * nt) | (ty << 16)), d.rho[gi],
-                        d.srho[gi]);
+      splitCoordinate(static_cast<double>(d.xcrd[gi]) * d.inv_gpos_scale, &hi.x, &lo.x);
+      splitCoordinate(static_cast<double>(d.ycrd[gi]) * d.inv_gpos_scale, &hi.y, &lo.y);
+      splitCoordinate(static_cast<double>(d.zcrd[gi]) * d.inv_gpos_scale, &hi.z, &lo.z);
       if (PASS == 2) {
-        pa.w = prm.x;
-        gbv.y = prm.y;      // the Lennard-Jones code, where pass 2 reads it
+        const int ty = d.lj_idx[gi];
+        w1 = d.charge[gi];
+        h = __int_as_float((ty * nt) | (ty << 16));
         if (GB) {
-          const float r = t.radius[gi];
-          pb.w = r;
-          gbv.x = 1.0f / r;
-        }
-        else {
-          pb.w = prm.z;
+          w2 = t.radius[gi];
+          g = 1.0f / w2;
         }
       }
       else {
-        pa.w = prm.w;
-        pb.w = prm.z;
+        w1 = d.srho[gi];
+        w2 = d.rho[gi];
         if (PASS == 3) {
-          gbv.y = t.sde[gi];
+          h = t.sde[gi];
         }
       }
     }
-    else {
-      pa = make_float4(5000.0f + 16.0f * static_cast<float>(slot), 0.0f, 0.0f, 0.0f);
-      pb = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
-      prm = make_float4(0.0f, __int_as_float(0), 1.0f, 0.0f);
+    putSlot(v, slot, hi, lo, w1, w2, g, h);
+    if (PASS != 2) {
+      v.neck[slot] = (d.neck_size > 0 && a < natom) ? d.neck_idx[base + a] : 0;
     }
-    v.pa[slot] = pa;
-    v.pb[slot] = pb;
-    v.prm[slot] = prm;
-    v.gbv[slot] = gbv;
-    v.neck[slot] = (d.neck_size > 0 && a < natom) ? d.neck_idx[base + a] : 0;
   }
   __syncwarp();
 }
 
-__device__ __forceinline__ UnitSmem warpView(float4* pa, float4* pb, float4* prm, float2* gbv,
-                                             int* neck, const float2* lj) {
+// A warp's slice of a tile kernel's shared memory
+struct TileStage {
+  float4 rec[kTiledWarps][5][kStageSlots / 2];
+  int neck[kTiledWarps][kStageSlots];
+  unsigned short late[kTiledWarps][kLateEntries];
+};
+
+__device__ __forceinline__ UnitSmem warpView(TileStage &m, const float2* lj) {
   UnitSmem v{};
   const int w = threadIdx.x >> 5;
-  v.pa = pa + w * kStageSlots;
-  v.pb = pb + w * kStageSlots;
-  v.prm = prm + w * kStageSlots;
-  v.gbv = gbv + w * kStageSlots;
-  v.neck = neck + w * kStageSlots;
+  v.pa = m.rec[w][0];
+  v.pb = m.rec[w][1];
+  v.pc = m.rec[w][2];
+  v.pd = m.rec[w][3];
+  v.pg = m.rec[w][4];
+  v.neck = m.neck[w];
+  v.late = m.late[w];
   v.lj = const_cast<float2*>(lj);
   return v;
 }
@@ -218,44 +189,44 @@ __device__ __forceinline__ void addGlobal(long long* acc, float v) {
 template <bool NECK>
 __global__ void __launch_bounds__(256, 4)
 kTiledRadii(const DevSynthesis d, const DevTiled t, int tile_begin, int tile_end) {
-  __shared__ float4 pa[kTiledWarps * kStageSlots], pb[kTiledWarps * kStageSlots];
-  __shared__ float4 prm[kTiledWarps * kStageSlots];
-  __shared__ float2 gbv[kTiledWarps * kStageSlots];
-  __shared__ int neck[kTiledWarps * kStageSlots];
+  __shared__ TileStage stage;
   const int lane = threadIdx.x & 31;
   const float ps = static_cast<float>(1 << kPsiBits);
   int first, last;
   warpTileRange(t, tile_begin, tile_end, &first, &last);
-  const UnitSmem v = warpView(pa, pb, prm, gbv, neck, d.ljab);
-  RadiiPass2<NECK> p(v, d);
+  const UnitSmem v = warpView(stage, d.ljab);
+  RadiiPass<false, NECK, true> p(v, d);
   for (int g = first; g < last; g++) {
     const int m = tiledOwner(t, g);
     const int sysid = t.systems[m];
     int I, J;
     const TileInfo ti = tiledTileInfo(d, sysid, g - t.tile_prefix[m], &I, &J);
     stageTile<1, true>(d, t, v, sysid, I, J, ti.diag, lane);
-    p.begin(lane);
-    walkTile2(p, ti, lane);
-    const int base = d.atom_start[sysid];
-    if (lane < ti.ni) {
-      addGlobal(&t.psi_acc[base + I * kTile + lane], p.psi_i * ps);
+    const TileWalk w = tileWalk(ti, lane);
+    p.begin(ti, w);
+    walkTile(p, ti, w, lane);
+    const int ia = d.atom_start[sysid] + I * kTile, ja = d.atom_start[sysid] + J * kTile;
+    const float vi = iShare(p.psi_i, w);
+    const float vj = jShare(p.psi_j, w, lane);
+    if (ownsAtom(ti, w, lane)) {
+      addGlobal(&t.psi_acc[ia + lane], vi * ps);
     }
-    const int jl = traveledAtom2(ti, lane);
+    const int jl = sharedAtom(w, lane);
     if (jl < ti.nj) {
-      addGlobal(&t.psi_acc[base + J * kTile + jl], p.psi_j1 * ps);
+      addGlobal(&t.psi_acc[ja + jl], vj * ps);
     }
+    p.finish(ti, lane, v.late, nullptr, [&](int slot, float x) {
+      addGlobal(&t.psi_acc[slot < kTile ? ia + slot : ja + slot - kTile], x * ps);
+    });
     __syncwarp();
   }
 }
 
 // Pass 2 (Coulomb + Lennard-Jones and GB pair terms) over tiles [tile_begin, tile_end)
 template <bool FORCE, bool ENERGY, bool NB, bool GB, bool CLASH>
-__global__ void __launch_bounds__(256, 4)
+__global__ void __launch_bounds__(256, 3)
 kTiledPair(const DevSynthesis d, const DevTiled t, int tile_begin, int tile_end) {
-  __shared__ float4 pa[kTiledWarps * kStageSlots], pb[kTiledWarps * kStageSlots];
-  __shared__ float4 prm[kTiledWarps * kStageSlots];
-  __shared__ float2 gbv[kTiledWarps * kStageSlots];
-  __shared__ int neck[kTiledWarps * kStageSlots];
+  __shared__ TileStage stage;
   const int lane = threadIdx.x & 31;
   const float fs = d.frc_scale;
   const float es = d.nrg_scale;
@@ -288,13 +259,14 @@ kTiledPair(const DevSynthesis d, const DevTiled t, int tile_begin, int tile_end)
     }
     int I, J;
     const TileInfo ti = tiledTileInfo(d, sysid, g - t.tile_prefix[m], &I, &J);
-    const UnitSmem v = warpView(pa, pb, prm, gbv, neck, d.ljab + d.lj_start[sysid]);
+    const UnitSmem v = warpView(stage, d.ljab + d.lj_start[sysid]);
     stageTile<2, GB>(d, t, v, sysid, I, J, ti.diag, lane);
+    const TileWalk w = tileWalk(ti, lane);
     unsigned mask = 0u;
     if (NB) {
       const int midx = d.tile_mask_idx[d.tile_start[sysid] + ti.local];
       if (midx != 0) {
-        mask = __ldg(&d.mask_pool[static_cast<size_t>(midx) * 32 + lane]);
+        mask = __ldg(&d.mask_pool[static_cast<size_t>(midx) * 32 + w.il]);
       }
     }
     PairPass<FORCE, ENERGY, NB, GB, CLASH> p(v, d.kappa, d.inv_dielectric);
@@ -303,27 +275,31 @@ kTiledPair(const DevSynthesis d, const DevTiled t, int tile_begin, int tile_end)
       const int cycle = (d.clash_cycle != nullptr) ? d.clash_cycle[sysid] : -1;
       clash = clashScaled(d.clash_distance, d.clash_ratio, d.clash_cycles, cycle);
     }
-    p.begin(lane, mask, clash);
-    walkTile(p, ti, lane);
-    const int base = d.atom_start[sysid];
+    p.begin(ti, w, mask, clash);
+    walkTile(p, ti, w, lane);
     if (FORCE) {
-      if (lane < ti.ni) {
-        const int gi = base + I * kTile + lane;
-        addGlobal(&d.xfrc[gi], p.fxi * fs);
-        addGlobal(&d.yfrc[gi], p.fyi * fs);
-        addGlobal(&d.zfrc[gi], p.fzi * fs);
+      const float fxi = iShare(p.fxi, w), fyi = iShare(p.fyi, w), fzi = iShare(p.fzi, w);
+      const float dei = GB ? iShare(p.dei, w) : 0.0f;
+      const float fxj = jShare(p.fxj, w, lane), fyj = jShare(p.fyj, w, lane);
+      const float fzj = jShare(p.fzj, w, lane);
+      const float dej = GB ? jShare(p.dej, w, lane) : 0.0f;
+      if (ownsAtom(ti, w, lane)) {
+        const int gi = d.atom_start[sysid] + I * kTile + lane;
+        addGlobal(&d.xfrc[gi], fxi * fs);
+        addGlobal(&d.yfrc[gi], fyi * fs);
+        addGlobal(&d.zfrc[gi], fzi * fs);
         if (GB) {
-          addGlobal(&t.de_acc[gi], p.dei * ds);
+          addGlobal(&t.de_acc[gi], dei * ds);
         }
       }
-      const int jl = traveledAtom(ti, lane);
+      const int jl = sharedAtom(w, lane);
       if (jl < ti.nj) {
-        const int gj = base + J * kTile + jl;
-        addGlobal(&d.xfrc[gj], p.fxj * fs);
-        addGlobal(&d.yfrc[gj], p.fyj * fs);
-        addGlobal(&d.zfrc[gj], p.fzj * fs);
+        const int gj = d.atom_start[sysid] + J * kTile + jl;
+        addGlobal(&d.xfrc[gj], -fxj * fs);
+        addGlobal(&d.yfrc[gj], -fyj * fs);
+        addGlobal(&d.zfrc[gj], -fzj * fs);
         if (GB) {
-          addGlobal(&t.de_acc[gj], p.dej * ds);
+          addGlobal(&t.de_acc[gj], dej * ds);
         }
       }
     }
@@ -347,15 +323,12 @@ kTiledPair(const DevSynthesis d, const DevTiled t, int tile_begin, int tile_end)
 template <bool NECK>
 __global__ void __launch_bounds__(256, 4)
 kTiledDeriv(const DevSynthesis d, const DevTiled t, int tile_begin, int tile_end) {
-  __shared__ float4 pa[kTiledWarps * kStageSlots], pb[kTiledWarps * kStageSlots];
-  __shared__ float4 prm[kTiledWarps * kStageSlots];
-  __shared__ float2 gbv[kTiledWarps * kStageSlots];
-  __shared__ int neck[kTiledWarps * kStageSlots];
+  __shared__ TileStage stage;
   const int lane = threadIdx.x & 31;
   const float fs = d.frc_scale;
   int first, last;
   warpTileRange(t, tile_begin, tile_end, &first, &last);
-  const UnitSmem v = warpView(pa, pb, prm, gbv, neck, d.ljab);
+  const UnitSmem v = warpView(stage, d.ljab);
   DerivPass<NECK> p(v, d);
   for (int g = first; g < last; g++) {
     const int m = tiledOwner(t, g);
@@ -363,22 +336,28 @@ kTiledDeriv(const DevSynthesis d, const DevTiled t, int tile_begin, int tile_end
     int I, J;
     const TileInfo ti = tiledTileInfo(d, sysid, g - t.tile_prefix[m], &I, &J);
     stageTile<3, true>(d, t, v, sysid, I, J, ti.diag, lane);
-    p.begin(lane);
-    walkTile(p, ti, lane);
-    const int base = d.atom_start[sysid];
-    if (lane < ti.ni) {
-      const int gi = base + I * kTile + lane;
-      addGlobal(&d.xfrc[gi], p.fxi * fs);
-      addGlobal(&d.yfrc[gi], p.fyi * fs);
-      addGlobal(&d.zfrc[gi], p.fzi * fs);
+    const TileWalk w = tileWalk(ti, lane);
+    p.begin(ti, w);
+    walkTile(p, ti, w, lane);
+    const int ia = d.atom_start[sysid] + I * kTile, ja = d.atom_start[sysid] + J * kTile;
+    const auto add = [&](int gi, float fx, float fy, float fz) {
+      addGlobal(&d.xfrc[gi], fx * fs);
+      addGlobal(&d.yfrc[gi], fy * fs);
+      addGlobal(&d.zfrc[gi], fz * fs);
+    };
+    const float fxi = iShare(p.fxi, w), fyi = iShare(p.fyi, w), fzi = iShare(p.fzi, w);
+    const float fxj = jShare(p.fxj, w, lane), fyj = jShare(p.fyj, w, lane);
+    const float fzj = jShare(p.fzj, w, lane);
+    if (ownsAtom(ti, w, lane)) {
+      add(ia + lane, -fxi, -fyi, -fzi);
     }
-    const int jl = traveledAtom(ti, lane);
+    const int jl = sharedAtom(w, lane);
     if (jl < ti.nj) {
-      const int gj = base + J * kTile + jl;
-      addGlobal(&d.xfrc[gj], p.fxj * fs);
-      addGlobal(&d.yfrc[gj], p.fyj * fs);
-      addGlobal(&d.zfrc[gj], p.fzj * fs);
+      add(ja + jl, fxj, fyj, fzj);
     }
+    p.finish(ti, lane, v.late, [&](int slot, float fx, float fy, float fz) {
+      add(slot < kTile ? ia + slot : ja + slot - kTile, fx, fy, fz);
+    });
     __syncwarp();
   }
 }

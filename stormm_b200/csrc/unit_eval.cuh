@@ -17,18 +17,27 @@
 //   pass 3      radius chain-rule forces (nonbonded_potential.tpp:1022-1290)
 //   commit      forces into the int64 + int32-overflow arrays, energies into per-system slots
 //
-// Pair passes walk 32 x 32 tiles of a molecule's lower triangle, one tile per warp.  Lane l
-// holds atom i = I*32 + l in registers; j atoms rotate through the lanes (lane l meets atom
-// (l + k) mod 32 of block J at step k) and j-side accumulators travel with a shuffle per step.
-// Diagonal tiles take 16 steps, the last one on half the lanes, so every pair is visited once.
-// Forces, psi and dE/dR leave registers once per tile through integer shared-memory atomics,
-// so every sum is independent of scheduling and the results are bit-identical run to run.
+// Pair passes walk 32 x 32 tiles of a molecule's lower triangle, one tile per warp, two pairs per
+// lane and step in packed FP32 (FFMA2 and kin).  A block's 32 atoms are held as 16 records of two
+// atoms q and q + 16; lane l holds atom i in registers, meets record (l + k) mod 16 at step k, and
+// the accumulators of a record's two j atoms travel with it through the 16 lanes of the half warp
+// (walkTile).  A tile whose block I has at most 16 atoms takes half the steps, both half warps
+// holding those atoms.  Forces, psi and dE/dR leave registers once per tile through integer
+// shared-memory atomics, so every sum is independent of scheduling and the results are
+// bit-identical run to run.
 //
-// Shared memory per atom slot: pos_a = (x_hi, y_hi, z_hi, w1) and pos_b = (x_lo, y_lo, z_lo, w2)
-// feed the pair passes with two 16-byte loads per partner; w1 / w2 carry what the pass needs
-// (pass 1 and 3: s*rho and rho; pass 2: charge and effective radius).  prm holds the static
-// per-atom values, gbv the reciprocal effective radius with the Lennard-Jones code (pass 2) and
-// then the chain-rule dE/dR (pass 3).
+// What bounds the passes is instruction issue.  Against one pair a lane and step from 16-byte
+// records per atom, the packed form issues about half the FP32 instructions per pair, and a half
+// warp reads 16 records of 16 bytes where 32 lanes read 32: half the shared-memory wavefronts.
+// With the branch-free descreening of hctSeries2: 1,024 molecules of 16-256 atoms, force + energy
+// with its copies, 445 -> 391 us; 60 minimization cycles of 4,096 molecules of 24-96 atoms 61.5 ->
+// 50.7 ms; 32 chains of 2,000-5,000 atoms 1,817 -> 1,600 us.
+//
+// Shared memory per atom pair record: pa = (x, x', y, y'), pb = (z, z', w1, w1'), pc = (lo x, lo x',
+// lo y, lo y'), pd = (lo z, lo z', w2, w2') and pg = (g, g', h, h'), where w1 / w2 carry what the
+// pass needs (pass 1 and 3: s*rho and rho; pass 2: charge and effective radius), g the reciprocal
+// effective radius and h the Lennard-Jones code bits (pass 2) or the chain-rule dE/dR (pass 3).
+// prm holds the static per-atom values.
 #ifndef STORMM_B200_UNIT_EVAL_CUH
 #define STORMM_B200_UNIT_EVAL_CUH
 
@@ -212,139 +221,131 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __
 
 
 // HCT descreening of an atom of offset radius rho by a neighbour of screened radius sj at
-// distance r (invr = 1/r), for two (r, rho, sj) combinations at once in packed FP32; returns the
-// amounts psi decreases by.
+// distance r (invr = 1/r): the amounts psi decreases by, and their radial derivative factors
+// -(1/r) dI/dr, for two pairs at once in packed FP32.
 //
-// Beyond r = 4 sj the reference's Taylor series applies (nonbonded_potential.tpp:590-596).
-// Closer in, the three closed forms the reference selects by overlap case (no overlap, partial
-// overlap, atom inside the neighbour's sphere: nonbonded_potential.tpp:597-628) are one
-// expression in U = r + sj and L = max(rho, |r - sj|):
+// Beyond r = 4 sj the reference's Taylor series applies (nonbonded_potential.tpp:590-596,
+// 1116-1121): with t = (sj / r)^2, the first five terms of
+//   I = (sj t / r^2) sum_k k / (2k + 1) t^(k-1),
+//   -(1/r) dI/dr = (sj t / r^4) sum_k k (2k + 2) / (2k + 1) t^(k-1).
+// Closer in, while the spheres do not overlap (r > rho + sj), the reference's closed form
+// (:597-604, :1122-1128) is the same series summed to infinity.  hctSeries2 takes both: five
+// terms, plus t^5 times a polynomial in t for the rest of the series where r <= 4 sj (weighted
+// minimax fits on 1/16 <= t <= 0.3: relative error of the sums below 1.1e-8 and 4.3e-9).  No
+// reciprocal, logarithm or cancellation, so it is more accurate than the closed form in FP32.
+// It tells where it does not apply (overlapping spheres, or t > 0.3): bonded neighbours mostly, a
+// few pairs per atom, which hctClosed2 evaluates after the tile's walk.  Against one
+// branch per step on r <= 4 sj (nearly every step of a small molecule has such a pair on some
+// lane): HCT_NOTE
+// BRANCH: the polynomial behind a branch, for tiles where most steps have no pair within 4 sj.
+constexpr float kSeriesLimit = 0.3f;
+
+struct Near2 {
+  bool x, y;
+};
+
+template <bool DERIV, bool BRANCH>
+__device__ __forceinline__ Near2 hctSeries2(float2 r, float2 invr, float2 rho, float2 sj,
+                                            float2* integral, float2* deriv) {
+  const float2 invr2 = mul2(invr, invr);
+  const float2 t = mul2(mul2(sj, sj), invr2);
+  const float2 touch = add2(rho, sj);
+  const bool near_x = t.x > 0.0625f;
+  const bool near_y = t.y > 0.0625f;
+  float2 ti = f2(0.0f), td = f2(0.0f);
+  if (!BRANCH || near_x || near_y) {
+    ti = fma2(t, f2(1.4148261547e0f), f2(7.0001393557e-2f));
+    ti = fma2(t, ti, f2(5.3365993500e-1f));
+    ti = fma2(t, ti, f2(4.5760014653e-1f));
+    ti = f2(near_x ? ti.x : 0.0f, near_y ? ti.y : 0.0f);
+    if (DERIV) {
+      td = fma2(t, f2(4.3931625366e1f), f2(-9.4689912796e0f));
+      td = fma2(t, td, f2(1.3106045723e1f));
+      td = fma2(t, td, f2(6.9396967888e0f));
+      td = fma2(t, td, f2(6.4842333794e0f));
+      td = f2(near_x ? td.x : 0.0f, near_y ? td.y : 0.0f);
+    }
+  }
+  ti = fma2(t, ti, f2(kTaylorDD));
+  ti = fma2(t, ti, f2(kTaylorD));
+  ti = fma2(t, ti, f2(kTaylorC));
+  ti = fma2(t, ti, f2(kTaylorB));
+  ti = fma2(t, ti, f2(kTaylorA));
+  const float2 scale = mul2(mul2(sj, t), invr2);
+  *integral = mul2(scale, ti);
+  if (DERIV) {
+    td = fma2(t, td, f2(kTaylorHH));
+    td = fma2(t, td, f2(kTaylorH));
+    td = fma2(t, td, f2(kTaylorG));
+    td = fma2(t, td, f2(kTaylorF));
+    td = fma2(t, td, f2(kTaylorE));
+    *deriv = mul2(mul2(scale, invr2), td);
+  }
+  // written so that a distance that is not a number is left to the closed forms, as before
+  return Near2{!(r.x > touch.x && t.x <= kSeriesLimit), !(r.y > touch.y && t.y <= kSeriesLimit)};
+}
+
+// The same from the closed forms, for both directions of one pair at any distance.  The three the
+// reference selects by overlap case
+// (no overlap, partial overlap, atom inside the neighbour's sphere: nonbonded_potential.tpp:
+// 597-628) are one expression in U = r + sj and L = max(rho, |r - sj|):
 //   I = 1/2 [1/L - 1/U + (sj^2 - r^2)/(4r) (1/L^2 - 1/U^2) + ln(L/U) / (2r)]
 //       + (1/rho - 1/L) when rho < sj - r,
-// and I = 0 when rho >= U.  One formula instead of four keeps a warp on at most two paths; the
-// inside case is rare, so a branch there beats a reciprocal per pair.  The closed form cancels
-// to a small remainder near r = 4 sj, so ln(L / U) needs an accurate absolute value: the fast
-// hardware logarithm (__logf) errs by about 1e-7 absolute with a consistent sign, which biased
-// every atom's psi by -6.5e-7 relative and the GB energy by +1.1e-6 relative (1,024 molecules
-// of 16-256 atoms); logf removes the bias (psi -7.6e-8, GB energy 1.0e-7).
-__device__ __forceinline__ float2 hctIntegral2(float2 r, float2 r2, float2 invr, float2 rho,
-                                               float2 sj) {
-  const bool far_x = r.x > 4.0f * sj.x;
-  const bool far_y = r.y > 4.0f * sj.y;
-  float2 vf = f2(0.0f);
-  float2 vn = f2(0.0f);
-  if (far_x || far_y) {
-    const float2 invr2 = mul2(invr, invr);
-    const float2 t = mul2(mul2(sj, sj), invr2);
-    float2 dumbo = fma2(t, f2(kTaylorDD), f2(kTaylorD));
-    dumbo = fma2(t, dumbo, f2(kTaylorC));
-    dumbo = fma2(t, dumbo, f2(kTaylorB));
-    dumbo = fma2(t, dumbo, f2(kTaylorA));
-    vf = mul2(mul2(mul2(sj, t), invr2), dumbo);
-  }
-  if (!(far_x && far_y)) {
-    const float2 u = add2(r, sj);
-    const float2 rms = sub2(r, sj);
-    const float2 l = f2(fmaxf(rho.x, fabsf(rms.x)), fmaxf(rho.y, fabsf(rms.y)));
-    const float2 lu = mul2(l, u);
-    const float2 inv_lu = f2(__fdividef(1.0f, lu.x), __fdividef(1.0f, lu.y));
-    const float2 il = mul2(u, inv_lu);
-    const float2 iu = mul2(l, inv_lu);
-    const float2 dlu = sub2(il, iu);
-    const float2 liu = mul2(l, iu);
-    const float2 lg = f2(logf(liu.x), logf(liu.y));
-    const float2 q = mul2(mul2(mul2(f2(0.25f), sub2(mul2(sj, sj), r2)), invr), dlu);
-    float2 v = add2(fma2(q, add2(il, iu), dlu), mul2(mul2(f2(0.5f), invr), lg));
-    if (rho.x < -rms.x) {
-      v.x += 2.0f * (__fdividef(1.0f, rho.x) - il.x);
-    }
-    if (rho.y < -rms.y) {
-      v.y += 2.0f * (__fdividef(1.0f, rho.y) - il.y);
-    }
-    vn = f2((rho.x < u.x) ? 0.5f * v.x : 0.0f, (rho.y < u.y) ? 0.5f * v.y : 0.0f);
-  }
-  return f2(far_x ? vf.x : vn.x, far_y ? vf.y : vn.y);
-}
-
-// Radial derivative of the HCT integral, -(1/r) dI/dr, the factor the reference multiplies by
-// the chain-rule dE/dR (nonbonded_potential.tpp:1116-1165), from the same unified expression
-// (lambda = dL/dr: 1 without overlap, 0 on partial overlap, -1 inside the neighbour):
+// and I = 0 when rho >= U.  Its derivative (:1129-1165), lambda = dL/dr being 1 without overlap, 0
+// on partial overlap and -1 inside the neighbour, q = (sj^2 - r^2)/(4r) and q' = dq/dr:
 //   dI/dr = 1/2 [-lambda/L^2 + 1/U^2 + q'(1/L^2 - 1/U^2) + 2q (1/U^3 - lambda/L^3)
-//                + (lambda/L - 1/U - ln(L/U)/r) / (2r)] - 1/L^2 (inside),
-// q = (sj^2 - r^2)/(4r), q' = dq/dr.
-__device__ __forceinline__ float hctDerivative(float r, float r2, float invr, float rho,
-                                               float sj) {
-  const float invr2 = invr * invr;
-  if (r > 4.0f * sj) {
-    const float t = sj * sj * invr2;
-    const float dumbo = kTaylorE + t * (kTaylorF + t * (kTaylorG + t * (kTaylorH + t * kTaylorHH)));
-    return t * sj * invr2 * invr2 * dumbo;
-  }
-  const float u = r + sj;
-  const float rms = r - sj;
-  const float l = fmaxf(rho, fabsf(rms));
-  const float lam = (rms >= rho) ? 1.0f : ((-rms > rho) ? -1.0f : 0.0f);
-  const float inv_lu = __fdividef(1.0f, l * u);
-  const float il = u * inv_lu;
-  const float iu = l * inv_lu;
-  const float il2 = il * il;
-  const float iu2 = iu * iu;
-  const float q = 0.25f * (sj * sj - r2) * invr;
-  const float dq = -0.25f * fmaf(sj * sj, invr2, 1.0f);
-  float di = -lam * il2 + iu2 + dq * (il2 - iu2) + 2.0f * q * (iu2 * iu - lam * il2 * il) +
-             0.5f * invr * (lam * il - iu - invr * logf(l * iu));
-  di = 0.5f * di - ((-rms > rho) ? il2 : 0.0f);
-  return (rho < u) ? -di * invr : 0.0f;
-}
-
-// The HCT integral and its radial derivative together, for both directions of one pair (x for
-// (rho.x, sj.x), y for (rho.y, sj.y)): the Taylor forms share t = (sj / r)^2, the closed forms
-// share the reciprocals and the logarithm.
-__device__ __forceinline__ void hctBoth2(float r, float r2, float invr, float2 rho, float2 sj,
-                                         float2* integral, float2* deriv) {
+//                + (lambda/L - 1/U - ln(L/U)/r) / (2r)] - 1/L^2 (inside).
+// Returns (I.x, I.y, derivative factor .x, .y).  ln(L / U) needs an accurate absolute
+// value where the form cancels: the fast hardware logarithm (__logf) errs by about 1e-7 absolute
+// with a consistent sign, which biased every atom's psi by -6.5e-7 relative and the GB energy by
+// +1.1e-6 relative (1,024 molecules of 16-256 atoms); logf removes the bias.
+template <bool DERIV>
+__device__ __forceinline__ float4 hctClosed2(float r, float r2, float invr, float2 rho, float2 sj) {
   const float invr2 = invr * invr;
   const bool far_x = r > 4.0f * sj.x;
   const bool far_y = r > 4.0f * sj.y;
   const float2 sj2 = mul2(sj, sj);
-  float2 vfi = f2(0.0f), vfd = f2(0.0f), vni = f2(0.0f), vnd = f2(0.0f);
+  float2 vfi = f2(0.0f), vfd = f2(0.0f), vnd = f2(0.0f);
   if (far_x || far_y) {
     const float2 t = mul2(sj2, f2(invr2));
     float2 di = fma2(t, f2(kTaylorDD), f2(kTaylorD));
     di = fma2(t, di, f2(kTaylorC));
     di = fma2(t, di, f2(kTaylorB));
     di = fma2(t, di, f2(kTaylorA));
-    float2 dd = fma2(t, f2(kTaylorHH), f2(kTaylorH));
-    dd = fma2(t, dd, f2(kTaylorG));
-    dd = fma2(t, dd, f2(kTaylorF));
-    dd = fma2(t, dd, f2(kTaylorE));
     const float2 tsr = mul2(mul2(sj, t), f2(invr2));
     vfi = mul2(tsr, di);
-    vfd = mul2(mul2(tsr, f2(invr2)), dd);
+    if (DERIV) {
+      float2 dd = fma2(t, f2(kTaylorHH), f2(kTaylorH));
+      dd = fma2(t, dd, f2(kTaylorG));
+      dd = fma2(t, dd, f2(kTaylorF));
+      dd = fma2(t, dd, f2(kTaylorE));
+      vfd = mul2(mul2(tsr, f2(invr2)), dd);
+    }
   }
-  if (!(far_x && far_y)) {
-    const float2 u = add2(f2(r), sj);
-    const float2 rms = sub2(f2(r), sj);
-    const float2 l = f2(fmaxf(rho.x, fabsf(rms.x)), fmaxf(rho.y, fabsf(rms.y)));
-    const bool in_x = -rms.x > rho.x;      // inside the neighbour's sphere
-    const bool in_y = -rms.y > rho.y;
-    const float2 lu = mul2(l, u);
-    const float2 inv_lu = f2(__fdividef(1.0f, lu.x), __fdividef(1.0f, lu.y));
-    const float2 il = mul2(u, inv_lu);
-    const float2 iu = mul2(l, inv_lu);
-    const float2 liu = mul2(l, iu);
-    const float2 lg = f2(logf(liu.x), logf(liu.y));
-    const float2 s2mr2 = sub2(sj2, f2(r2));
-    // the integral
-    const float2 dlu = sub2(il, iu);
-    const float2 q = mul2(mul2(f2(0.25f * invr), s2mr2), dlu);
-    float2 v = add2(fma2(q, add2(il, iu), dlu), mul2(f2(0.5f * invr), lg));
-    if (in_x) {
-      v.x += 2.0f * (__fdividef(1.0f, rho.x) - il.x);
-    }
-    if (in_y) {
-      v.y += 2.0f * (__fdividef(1.0f, rho.y) - il.y);
-    }
-    vni = f2((rho.x < u.x) ? 0.5f * v.x : 0.0f, (rho.y < u.y) ? 0.5f * v.y : 0.0f);
+  const float2 u = add2(f2(r), sj);
+  const float2 rms = sub2(f2(r), sj);
+  const float2 l = f2(fmaxf(rho.x, fabsf(rms.x)), fmaxf(rho.y, fabsf(rms.y)));
+  const bool in_x = -rms.x > rho.x;      // inside the neighbour's sphere
+  const bool in_y = -rms.y > rho.y;
+  const float2 lu = mul2(l, u);
+  const float2 inv_lu = f2(__fdividef(1.0f, lu.x), __fdividef(1.0f, lu.y));
+  const float2 il = mul2(u, inv_lu);
+  const float2 iu = mul2(l, inv_lu);
+  const float2 liu = mul2(l, iu);
+  const float2 lg = f2(logf(liu.x), logf(liu.y));
+  const float2 s2mr2 = sub2(sj2, f2(r2));
+  // the integral
+  const float2 dlu = sub2(il, iu);
+  const float2 q = mul2(mul2(f2(0.25f * invr), s2mr2), dlu);
+  float2 v = add2(fma2(q, add2(il, iu), dlu), mul2(f2(0.5f * invr), lg));
+  if (in_x) {
+    v.x += 2.0f * (__fdividef(1.0f, rho.x) - il.x);
+  }
+  if (in_y) {
+    v.y += 2.0f * (__fdividef(1.0f, rho.y) - il.y);
+  }
+  const float2 vni = f2((rho.x < u.x) ? 0.5f * v.x : 0.0f, (rho.y < u.y) ? 0.5f * v.y : 0.0f);
+  if (DERIV) {
     // its derivative, lambda = dL/dr
     const float2 lam = f2((rms.x >= rho.x) ? 1.0f : (in_x ? -1.0f : 0.0f),
                           (rms.y >= rho.y) ? 1.0f : (in_y ? -1.0f : 0.0f));
@@ -361,8 +362,8 @@ __device__ __forceinline__ void hctBoth2(float r, float r2, float invr, float2 r
     const float2 w = mul2(dv, f2(-invr));
     vnd = f2((rho.x < u.x) ? w.x : 0.0f, (rho.y < u.y) ? w.y : 0.0f);
   }
-  *integral = f2(far_x ? vfi.x : vni.x, far_y ? vfi.y : vni.y);
-  *deriv = f2(far_x ? vfd.x : vnd.x, far_y ? vfd.y : vnd.y);
+  return make_float4(far_x ? vfi.x : vni.x, far_y ? vfi.y : vni.y, far_x ? vfd.x : vnd.x,
+                     far_y ? vfd.y : vnd.y);
 }
 
 // Neck GB (Mongan's neck between two spheres, nonbonded_potential.tpp:678-702, 1219-1245): pairs
@@ -384,7 +385,7 @@ struct NeckGb {
     const float m2 = m * m;
     return __fdividef(scale * __ldg(&val[t]), 1.0f + m2 + 0.3f * m2 * m2 * m2);
   }
-  // the same and its radial derivative factor -(1/r) dI/dr, as hctDerivative
+  // the same and its radial derivative factor -(1/r) dI/dr
   __device__ __forceinline__ float both(int ni, int nj, float r, float invr, float* deriv) const {
     const int t = size * nj + ni;
     const float m = r - __ldg(&sep[t]);
@@ -398,11 +399,13 @@ struct NeckGb {
 
 // Shared-memory layout of one work unit
 struct UnitSmem {
-  float4* pa;       // x_hi, y_hi, z_hi, pass payload w1
-  float4* pb;       // x_lo, y_lo, z_lo, pass payload w2
+  float4* pa;       // x, y (hi parts) of the record's two atoms
+  float4* pb;       // z (hi), pass payload w1
+  float4* pc;       // x, y (lo parts)
+  float4* pd;       // z (lo), pass payload w2
+  float4* pg;       // 1 / effective radius; Lennard-Jones code bits in pass 2, dE/dR after the
+                    // chain rule
   float4* prm;      // charge * sqrt(k_Coulomb), Lennard-Jones code (int bits), rho, s * rho
-  float2* gbv;      // 1 / effective radius; y: Lennard-Jones code bits in pass 2, dE/dR after
-                    // the chain rule
   int* fx;          // int63 force accumulators: primary
   int* fy;
   int* fz;
@@ -425,7 +428,19 @@ struct UnitSmem {
   int* achunk0;
   int* dchunk0;
   float2* clash;    // per unit molecule: clash distance and sigma ratio of this evaluation
+  unsigned short* late;   // kLateEntries per warp: pairs of GB pass 1 set aside (RadiiPass)
 };
+
+// Atom pair records: slot s of a unit is atom (s / 16) % 2 of record 16 (s / 32) + s % 16
+constexpr int kRecords = kTile / 2;
+__device__ __forceinline__ int slotRecord(int slot) {
+  return (slot >> 5) * kRecords + (slot & (kRecords - 1));
+}
+__device__ __forceinline__ int slotHalf(int slot) { return (slot >> 4) & 1; }
+// Component c (0: first pair, 2: second pair) of a slot in a record array
+__device__ __forceinline__ float &slotValue(float4* a, int slot, int c) {
+  return reinterpret_cast<float*>(a)[4 * slotRecord(slot) + c + slotHalf(slot)];
+}
 
 __host__ __device__ inline size_t alignUp(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
@@ -460,7 +475,9 @@ cudaError_t allowLargeSmem(K kern) {
   return err;
 }
 
-constexpr int kSlotBytes = 3 * 16 + 8 + 11 * 4;
+constexpr int kSlotBytes = 5 * 8 + 16 + 11 * 4;
+constexpr int kLateEntries = 128;   // per warp: pairs of a tile set aside before they are evaluated
+constexpr int kLateWarps = 16;      // warps of the largest block
 
 // Dynamic shared memory of one work unit's evaluation: max_slots atom slots, max_lj table entries
 __host__ __device__ inline size_t unitSmemBytes(int max_slots, int max_lj,
@@ -472,6 +489,7 @@ __host__ __device__ inline size_t unitSmemBytes(int max_slots, int max_lj,
   b += sizeof(unsigned long long) * max_sys * kNrgStride;
   b += sizeof(float2) * max_sys;
   b += sizeof(int) * (3 * max_sys + 5 * (max_sys + 1));
+  b += sizeof(unsigned short) * kLateEntries * kLateWarps;
   return alignUp(b, 16);
 }
 
@@ -479,10 +497,13 @@ __device__ UnitSmem carveSmem(char* base, int max_slots, int max_lj,
                               int max_sys = kMaxUnitSystems) {
   UnitSmem s;
   size_t off = 0;
-  s.pa = reinterpret_cast<float4*>(base + off); off += sizeof(float4) * max_slots;
-  s.pb = reinterpret_cast<float4*>(base + off); off += sizeof(float4) * max_slots;
+  const size_t records = sizeof(float4) * (max_slots / 2);
+  s.pa = reinterpret_cast<float4*>(base + off); off += records;
+  s.pb = reinterpret_cast<float4*>(base + off); off += records;
+  s.pc = reinterpret_cast<float4*>(base + off); off += records;
+  s.pd = reinterpret_cast<float4*>(base + off); off += records;
+  s.pg = reinterpret_cast<float4*>(base + off); off += records;
   s.prm = reinterpret_cast<float4*>(base + off); off += sizeof(float4) * max_slots;
-  s.gbv = reinterpret_cast<float2*>(base + off); off += sizeof(float2) * max_slots;
   int* ip = reinterpret_cast<int*>(base + off);
   s.fx = ip; ip += max_slots;
   s.fy = ip; ip += max_slots;
@@ -511,11 +532,11 @@ __device__ UnitSmem carveSmem(char* base, int max_slots, int max_lj,
   s.bchunk0 = q; q += max_sys + 1;
   s.achunk0 = q; q += max_sys + 1;
   s.dchunk0 = q; q += max_sys + 1;
+  s.late = reinterpret_cast<unsigned short*>(q);
   return s;
 }
 
-// The threads that evaluate one work unit together: a whole block, or a single warp (small
-// molecules, where block-wide barriers would cost more than the work between them)
+// The threads that evaluate one work unit together: a whole block
 struct BlockTeam {
   __device__ __forceinline__ int rank() const { return threadIdx.x; }
   __device__ __forceinline__ int size() const { return blockDim.x; }
@@ -523,15 +544,6 @@ struct BlockTeam {
   __device__ __forceinline__ int warps() const { return blockDim.x >> 5; }
   __device__ __forceinline__ void sync() const { __syncthreads(); }
   __device__ __forceinline__ bool any(bool p) const { return __syncthreads_or(p) != 0; }
-};
-
-struct WarpTeam {
-  __device__ __forceinline__ int rank() const { return threadIdx.x & 31; }
-  __device__ __forceinline__ int size() const { return 32; }
-  __device__ __forceinline__ int warp() const { return 0; }
-  __device__ __forceinline__ int warps() const { return 1; }
-  __device__ __forceinline__ void sync() const { __syncwarp(); }
-  __device__ __forceinline__ bool any(bool p) const { return __any_sync(0xffffffffu, p) != 0; }
 };
 
 // Index of the unit molecule that owns position pos of a prefix-sum array of n + 1 entries
@@ -552,10 +564,19 @@ __device__ __forceinline__ void tileCoordinates(int local, int* ti, int* tj) {
   *tj = local - i * (i + 1) / 2;
 }
 
-__device__ __forceinline__ float3 pairDelta(const float4 a_i, const float4 b_i, const float4 a_j,
-                                            const float4 b_j) {
-  return make_float3((a_j.x - a_i.x) + (b_j.x - b_i.x), (a_j.y - a_i.y) + (b_j.y - b_i.y),
-                     (a_j.z - a_i.z) + (b_j.z - b_i.z));
+// High and low parts of a slot's coordinates
+__device__ __forceinline__ float3 slotHi(const UnitSmem &s, int slot) {
+  return make_float3(slotValue(s.pa, slot, 0), slotValue(s.pa, slot, 2), slotValue(s.pb, slot, 0));
+}
+__device__ __forceinline__ float3 slotLo(const UnitSmem &s, int slot) {
+  return make_float3(slotValue(s.pc, slot, 0), slotValue(s.pc, slot, 2), slotValue(s.pd, slot, 0));
+}
+
+// Coordinate difference b - a from the hi / lo representation of two slots
+__device__ __forceinline__ float3 slotDelta(const UnitSmem &s, int a, int b) {
+  const float3 ah = slotHi(s, a), al = slotLo(s, a), bh = slotHi(s, b), bl = slotLo(s, b);
+  return make_float3((bh.x - ah.x) + (bl.x - al.x), (bh.y - ah.y) + (bl.y - al.y),
+                     (bh.z - ah.z) + (bl.z - al.z));
 }
 
 __device__ __forceinline__ void addForce(const UnitSmem &s, int slot, float fx, float fy, float fz,
@@ -595,11 +616,6 @@ __device__ __forceinline__ void warpEnergy(const UnitSmem &s, int k, int slot, f
   }
 }
 
-// Coordinate difference b - a from the hi / lo representation of two slots
-__device__ __forceinline__ float3 slotDelta(const UnitSmem &s, int a, int b) {
-  return pairDelta(s.pa[a], s.pb[a], s.pa[b], s.pb[b]);
-}
-
 // ------------------------------------------------------------------------------------------------
 // Valence terms (Potential/valence_potential.tpp).  Warps take chunks of 32 terms of one molecule,
 // so each chunk's energies reduce across the warp into a single shared-memory update.
@@ -619,10 +635,8 @@ struct SmemValence {
       sys(s_in.sys), slot0(s_in.slot0), begin(begin_in), stride(stride_in) {}
   __device__ __forceinline__ int chunkBegin() const { return begin; }
   __device__ __forceinline__ int chunkStride() const { return stride; }
-  __device__ __forceinline__ float4 pa(int i) const { return s.pa[i]; }
-  __device__ __forceinline__ float4 pb(int i) const { return s.pb[i]; }
-  __device__ __forceinline__ float4 prm(int i) const { return s.prm[i]; }
-  __device__ __forceinline__ float3 delta(int a, int b) const { return slotDelta(s, a, b); }
+  __device__ __forceinline__ float3 hi(int i) const { return slotHi(s, i); }
+  __device__ __forceinline__ float3 lo(int i) const { return slotLo(s, i); }
   __device__ __forceinline__ void force(int i, float fx, float fy, float fz, float scale) const {
     addForce(s, i, fx, fy, fz, scale);
   }
@@ -631,8 +645,8 @@ struct SmemValence {
   }
   // exact coordinates of a slot: the hi + lo float pair summed in double
   __device__ __forceinline__ double3 pos64(int i) const {
-    const float4 a = s.pa[i];
-    const float4 b = s.pb[i];
+    const float3 a = slotHi(s, i);
+    const float3 b = slotLo(s, i);
     return make_double3(static_cast<double>(a.x) + static_cast<double>(b.x),
                         static_cast<double>(a.y) + static_cast<double>(b.y),
                         static_cast<double>(a.z) + static_cast<double>(b.z));
@@ -649,10 +663,6 @@ struct SmemValence {
     }
   }
   __device__ __forceinline__ float2 clash(int k) const { return s.clash[k]; }
-  // the molecule's 1-4 table follows its standard table in shared memory
-  __device__ __forceinline__ float2 lj14(int code_i, int code_l, int nt) const {
-    return s.lj[(code_i & 0xffff) + (code_l >> 16) + nt * nt];
-  }
 };
 
 template <bool FORCE, bool ENERGY, class V, bool CLASH = false>
@@ -676,7 +686,7 @@ __device__ void valenceTerms(const DevSynthesis &d, const V &v, int nsys_u) {
       const float keq = __uint_as_float(rec.y);
       const float leq_hi = __uint_as_float(rec.z);
       const float leq_lo = __uint_as_float(rec.w);
-      const float4 ai = v.pa(ia), aj = v.pa(ja), bi = v.pb(ia), bj = v.pb(ja);
+      const float3 ai = v.hi(ia), aj = v.hi(ja), bi = v.lo(ia), bj = v.lo(ja);
       const float av[3] = {aj.x, aj.y, aj.z};
       const float bv[3] = {ai.x, ai.y, ai.z};
       const float lav[3] = {bj.x, bj.y, bj.z};
@@ -938,182 +948,366 @@ __device__ __forceinline__ TileInfo tileInfo(const UnitSmem &s, int nsys_u, int 
   return ti;
 }
 
-// Run one tile: p.pair(jslot, jl) for every pair of the tile (once each) and p.rotate() after
-// every step.  Padding slots hold parameters that make every contribution to a real atom exactly
-// zero (no charge, zero screened radius and dE/dR, masked Lennard-Jones, far-away coordinates),
-// so partial tiles run the same branch-free loop; only the last step of a diagonal tile, where
-// lanes l and l + 16 would meet the same pair, runs on half the lanes.
+// How a warp walks a tile.  Lane l = 16 h + p holds atom il of block I and meets record
+// (q + k) mod 16 of block J at step k, that is atoms q and q + 16:
+//   off-diagonal                       il = l, q = p, 16 steps: all 32 atoms of block J
+//   off-diagonal, at most 16 atoms     il = p, q = p + 8 h, 8 steps: each half warp takes half of
+//   in block I                         the records
+//   diagonal                           il = l, q = p, 9 steps: a lane's own half of the block at
+//                                      distances 1 to 8, the other half at distances 0 to 7 (h = 0)
+//                                      or 1 to 8 (h = 1), so that every pair is met once
+//   diagonal, at most 16 atoms         il = p, q = p + 1 + 4 h, 4 steps: distances 1 to 4 (h = 0)
+//                                      and 5 to 8 (h = 1)
+// The traveling accumulators of a record pass from lane to lane within the half warp; after the
+// walk, `partner` is the lane of the other half that holds sums of the same record.
+struct TileWalk {
+  int il;
+  int q;
+  int steps;
+  int partner;
+  bool narrow;
+  bool diag;
+};
+
+__device__ __forceinline__ TileWalk tileWalk(const TileInfo &ti, int lane) {
+  const int p = lane & 15, h = lane >> 4;
+  TileWalk w;
+  w.diag = ti.diag;
+  w.narrow = ti.ni <= kRecords;
+  const int offset = w.narrow ? (ti.diag ? 1 + 4 * h : 8 * h) : 0;
+  const int ahead = w.narrow ? (ti.diag ? (h != 0 ? 4 : -4) : 8) : 0;
+  w.il = w.narrow ? p : lane;
+  w.q = (p + offset) & 15;
+  w.steps = w.narrow ? (ti.diag ? 4 : 8) : (ti.diag ? 9 : 16);
+  w.partner = ((h ^ 1) << 4) | ((p + ahead) & 15);
+  return w;
+}
+
+// Weights (1 or 0) of the two pairs of step k of a diagonal tile
+__device__ __forceinline__ float2 diagonalWeights(const TileWalk &w, int lane, int k) {
+  const int p = lane & 15, h = lane >> 4;
+  if (w.narrow) {
+    // atoms q + 16 are padding, which needs no mask
+    return f2((k == 3 && h == 1 && p >= 8) ? 0.0f : 1.0f, 1.0f);
+  }
+  if (k == 0) {
+    return f2(0.0f, h == 0 ? 1.0f : 0.0f);
+  }
+  if (k == 8) {
+    return f2((h == 1 || p < 8) ? 1.0f : 0.0f, (h == 1 && p < 8) ? 1.0f : 0.0f);
+  }
+  return f2(1.0f, 1.0f);
+}
+
+// Run one tile: p.pair<false>(record, q, 1) for every step, or p.pair<true>(record, q, weights)
+// where pairs of weight 0 are to be left out, and p.rotate(source lane) after it.  Padding slots
+// hold parameters that make every contribution to a real atom exactly zero (no charge, zero
+// screened radius and dE/dR, masked Lennard-Jones, far-away coordinates), so partial tiles run the
+// same branch-free loop.
 //
-// tileFlush(p) runs after every eighth step and at the end of the tile: passes that sum energies
-// in FP32 move their partial sums into integer accumulators there, so no FP32 running sum spans
-// more than eight pairs (the generic overload does nothing).
+// tileFlush(p) runs after at most eight steps and at the end of the tile: passes that sum energies
+// in FP32 move their partial sums into FP64 there, so no FP32 running sum spans more than eight
+// pairs of each of the two (the generic overload does nothing).
 template <class P>
 __device__ __forceinline__ void tileFlush(P &) {}
 
 template <class P>
-__device__ __forceinline__ void walkTile(P &p, const TileInfo &ti, int lane) {
-  if (!ti.diag) {
+__device__ __forceinline__ void walkTile(P &p, const TileInfo &ti, const TileWalk &w, int lane) {
+  const int jrec = slotRecord(ti.jbase);
+  const int src = (lane & 16) | ((lane + 1) & 15);
+  int q = w.q;
+  if (!w.diag) {
 #pragma unroll 1
-    for (int k0 = 0; k0 < kTile; k0 += 8) {
-#pragma unroll 2
-      for (int k = k0; k < k0 + 8; k++) {
-        const int jl = (lane + k) & 31;
-        p.pair(ti.jbase + jl, jl);
-        p.rotate(lane);
+    for (int k0 = 0; k0 < w.steps; k0 += 8) {
+#pragma unroll P::kUnroll
+      for (int k = 0; k < 8; k++) {
+        p.template pair<false>(jrec + q, q, f2(1.0f));
+        p.rotate(src);
+        q = (q + 1) & 15;
       }
       tileFlush(p);
     }
   }
   else {
 #pragma unroll 1
-    for (int k = 1; k < 16; k++) {
-      const int jl = (lane + k) & 31;
-      p.pair(ti.jbase + jl, jl);
-      p.rotate(lane);
-      if (k == 8) {
+    for (int k = 0; k < w.steps; k++) {
+      p.template pair<true>(jrec + q, q, diagonalWeights(w, lane, k));
+      p.rotate(src);
+      q = (q + 1) & 15;
+      if (k == 4) {
         tileFlush(p);
       }
     }
-    if (lane < 16) {
-      p.pair(ti.jbase + lane + 16, lane + 16);
-    }
-    p.rotate(lane);
     tileFlush(p);
   }
 }
 
-// Walk a tile two pairs per lane per step: an off-diagonal tile in 16 steps pairing j = l + k
-// with j = l + k + 16, a diagonal tile in 8 steps pairing j = l + k with j = l + k + 8 (the
-// second pair of the last step on half the lanes: w2 = 0 elsewhere).  Each of the two j streams
-// carries its own traveling accumulators; p.merge() folds the second into the first, after which
-// lane l holds those of block J's atom (l + 16) mod 32 (off-diagonal) or (l + 9) mod 32.
-template <class P>
-__device__ __forceinline__ void walkTile2(P &p, const TileInfo &ti, int lane) {
-  if (!ti.diag) {
-#pragma unroll 2
-    for (int k = 0; k < 16; k++) {
-      const int j1 = (lane + k) & 31;
-      const int j2 = (lane + k + 16) & 31;
-      p.pair2(ti.jbase + j1, j1, ti.jbase + j2, j2, 1.0f);
-      p.rotate2(lane);
-    }
-    p.merge((lane + 16) & 31);
+// Block J's atom whose traveling sum jShare() leaves with this lane after the walk
+__device__ __forceinline__ int sharedAtom(const TileWalk &w, int lane) {
+  return ((w.q + w.steps) & 15) + (lane & 16);
+}
+
+// The two half warps' sums of a record's two atoms: half h takes atom q + 16 h's
+__device__ __forceinline__ float jShare(float2 acc, const TileWalk &w, int lane) {
+  const bool upper = (lane & 16) != 0;
+  const float other = __shfl_sync(kFullMask, upper ? acc.x : acc.y, w.partner);
+  return (upper ? acc.y : acc.x) + other;
+}
+
+// Block I's atom's sum over a lane's two pairs, and over both half warps where both hold the atom
+// (the lanes of the lower half commit it)
+__device__ __forceinline__ float iShare(float2 acc, const TileWalk &w) {
+  const float v = acc.x + acc.y;
+  return w.narrow ? v + __shfl_xor_sync(kFullMask, v, 16) : v;
+}
+
+// Whether this lane commits block I's atom il
+__device__ __forceinline__ bool ownsAtom(const TileInfo &ti, const TileWalk &w, int lane) {
+  return lane < ti.ni && w.il == lane;
+}
+
+// Atom i's coordinates, negated and in both halves of a packed pair
+struct AtomI {
+  float2 hx, hy, hz, lx, ly, lz;
+  __device__ __forceinline__ void load(const UnitSmem &s, int slot) {
+    const float3 h = slotHi(s, slot), l = slotLo(s, slot);
+    hx = f2(-h.x);
+    hy = f2(-h.y);
+    hz = f2(-h.z);
+    lx = f2(-l.x);
+    ly = f2(-l.y);
+    lz = f2(-l.z);
   }
-  else {
-#pragma unroll 1
-    for (int k = 1; k <= 8; k++) {
-      const int j1 = (lane + k) & 31;
-      const int j2 = (lane + k + 8) & 31;
-      p.pair2(ti.jbase + j1, j1, ti.jbase + j2, j2, (k == 8 && lane >= 16) ? 0.0f : 1.0f);
-      p.rotate2(lane);
+};
+
+// Separations j - i of a record's two atoms, and their squares' sum; with GUARD, pairs of weight 0
+// are put 1e4 A apart
+struct Separation2 {
+  float2 hx, hy, hz, lx, ly, lz;   // of the hi and lo parts
+  float2 dx, dy, dz, r2;
+};
+
+template <bool GUARD>
+__device__ __forceinline__ Separation2 separate2(const AtomI &i, float4 a, float4 b, float4 c,
+                                                 float4 d, float2 w) {
+  Separation2 v;
+  v.hx = add2(f2(a.x, a.y), i.hx);
+  v.hy = add2(f2(a.z, a.w), i.hy);
+  v.hz = add2(f2(b.x, b.y), i.hz);
+  v.lx = add2(f2(c.x, c.y), i.lx);
+  v.ly = add2(f2(c.z, c.w), i.ly);
+  v.lz = add2(f2(d.x, d.y), i.lz);
+  v.dx = add2(v.hx, v.lx);
+  v.dy = add2(v.hy, v.ly);
+  v.dz = add2(v.hz, v.lz);
+  v.r2 = fma2(v.dx, v.dx, fma2(v.dy, v.dy, mul2(v.dz, v.dz)));
+  if (GUARD) {
+    v.r2 = f2(w.x != 0.0f ? v.r2.x : 1.0e8f, w.y != 0.0f ? v.r2.y : 1.0e8f);
+  }
+  return v;
+}
+
+// Pairs set aside by a pass, spread over the warp: every lane's bits in `late` (bit k for the
+// first pair of step k, bit 16 + k for the second) become entries lane | bit << 5 of the warp's
+// list, and f(lane, bit) runs for each, one a lane, so that the few pairs of a tile take one or
+// two rounds where lane by lane the busiest lane would set the count.
+template <class F>
+__device__ __forceinline__ void spreadLate(unsigned late, unsigned short* list, int lane,
+                                           const F &f) {
+  while (__any_sync(kFullMask, late != 0u)) {
+    const int mine = __popc(late);
+    int end = mine;                       // inclusive prefix sum over the lanes
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(kFullMask, end, o);
+      end += (lane >= o) ? v : 0;
     }
-    p.merge((lane + 24) & 31);
+    const int total = min(__shfl_sync(kFullMask, end, 31), kLateEntries);
+    for (int at = end - mine; late != 0u && at < kLateEntries; at++) {
+      const int b = __ffs(late) - 1;
+      late &= late - 1u;
+      list[at] = static_cast<unsigned short>(lane | (b << 5));
+    }
+    __syncwarp();
+    for (int e = lane; e < total; e += 32) {
+      f(list[e] & 31, list[e] >> 5);
+    }
+    __syncwarp();
   }
 }
 
-__device__ __forceinline__ int traveledAtom2(const TileInfo &ti, int lane) {
-  return (lane + (ti.diag ? 9 : 16)) & 31;
-}
+// Slots of a pair set aside by lane `of` at bit b, and its step
+struct LatePair {
+  int islot, jslot, step;
+  float2 rho, sj;      // (rho_i, rho_j), (s_j rho_j, s_i rho_i)
+  float r, r2, invr;
+  float3 dv;           // j - i
+  __device__ __forceinline__ LatePair(const UnitSmem &s, const TileInfo &ti, int of, int b) {
+    const TileWalk w = tileWalk(ti, of);
+    step = b & 15;
+    islot = ti.ibase + w.il;
+    jslot = ti.jbase + ((w.q + step) & 15) + (b & 16);
+    dv = slotDelta(s, islot, jslot);
+    r2 = fmaf(dv.x, dv.x, fmaf(dv.y, dv.y, dv.z * dv.z));
+    invr = rsqrtf(r2);
+    r = r2 * invr;
+    rho = f2(slotValue(s.pd, islot, 2), slotValue(s.pd, jslot, 2));
+    sj = f2(slotValue(s.pb, jslot, 2), slotValue(s.pb, islot, 2));
+  }
+};
 
-// Lane that holds block J's atom jl's traveling accumulator once the walk is over
-__device__ __forceinline__ int traveledAtom(const TileInfo &ti, int lane) {
-  return (lane + (ti.diag ? 17 : 32)) & 31;
-}
-
-// GB pass 1, two pairs per lane per step: psi_i -= H(r, rho_i, s_j rho_j) and
-// psi_j -= H(r, rho_j, s_i rho_i)
-template <bool NECK = false>
-struct RadiiPass2 {
+// GB pass 1: psi_i -= H(r, rho_i, s_j rho_j) and psi_j -= H(r, rho_j, s_i rho_i).  STORE (a force
+// evaluation of the fused kernel): the radial derivatives of both terms go to the store for pass 3,
+// one float4 per lane and step of the tile walk, so the stores of a step are one coalesced 512-byte
+// line.  Pairs that hctSeries2 leaves out are marked in `late` and evaluated by finish() after the
+// walk.
+template <bool STORE, bool NECK = false, bool BRANCH = false>
+struct RadiiPass {
+  static constexpr int kUnroll = 2;
   const UnitSmem &s;
   NeckGb neck;
-  float4 ai, bi;
-  int ni;           // neck index of atom i
-  float2 psi_i2;    // i-side sums of the two pair streams
-  float2 psi_j;     // traveling j-side sums: x for stream 1, y for stream 2
-  float psi_i, psi_j1;
-  __device__ RadiiPass2(const UnitSmem &s_in, const DevSynthesis &d) : s(s_in), neck(d) {}
-  __device__ __forceinline__ void begin(int islot) {
-    ai = s.pa[islot];
-    bi = s.pb[islot];
+  AtomI at;
+  float2 rho_i, s_i;    // radius and screened radius of atom i
+  int ni;               // neck index of atom i
+  int jneck;            // slot of block J's first atom
+  float2 psi_i, psi_j;  // i-side sums, traveling j-side sums
+  unsigned late, bit;   // pairs left to finish(), bit of the current step
+  float4* out;          // this lane's entry of the store for the current step
+  __device__ RadiiPass(const UnitSmem &s_in, const DevSynthesis &d) : s(s_in), neck(d) {}
+  __device__ __forceinline__ void begin(const TileInfo &ti, const TileWalk &w,
+                                        float4* tile_out = nullptr) {
+    const int islot = ti.ibase + w.il;
+    at.load(s, islot);
+    rho_i = f2(slotValue(s.pd, islot, 2));
+    s_i = f2(slotValue(s.pb, islot, 2));
     if (NECK) {
       ni = s.neck[islot];
+      jneck = ti.jbase;
     }
-    psi_i2 = f2(0.0f);
+    psi_i = f2(0.0f);
     psi_j = f2(0.0f);
+    late = 0u;
+    bit = 1u;
+    out = tile_out;
   }
-  __device__ __forceinline__ void pair2(int js1, int, int js2, int, float w2) {
-    const float4 aj1 = s.pa[js1];
-    const float4 bj1 = s.pb[js1];
-    const float4 aj2 = s.pa[js2];
-    const float4 bj2 = s.pb[js2];
-    const float2 dx = add2(sub2(f2(aj1.x, aj2.x), f2(ai.x)), sub2(f2(bj1.x, bj2.x), f2(bi.x)));
-    const float2 dy = add2(sub2(f2(aj1.y, aj2.y), f2(ai.y)), sub2(f2(bj1.y, bj2.y), f2(bi.y)));
-    const float2 dz = add2(sub2(f2(aj1.z, aj2.z), f2(ai.z)), sub2(f2(bj1.z, bj2.z), f2(bi.z)));
-    const float2 r2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
-    const float2 invr = f2(rsqrtf(r2.x), rsqrtf(r2.y));
-    const float2 r = mul2(r2, invr);
-    float2 hi = hctIntegral2(r, r2, invr, f2(bi.w), f2(aj1.w, aj2.w));
-    float2 hj = hctIntegral2(r, r2, invr, f2(bj1.w, bj2.w), f2(ai.w));
+  template <bool GUARD>
+  __device__ __forceinline__ void pair(int rec, int q, float2 wt) {
+    const float4 a = s.pa[rec], b = s.pb[rec], c = s.pc[rec], d = s.pd[rec];
+    const Separation2 v = separate2<GUARD>(at, a, b, c, d, wt);
+    const float2 invr = f2(rsqrtf(v.r2.x), rsqrtf(v.r2.y));
+    const float2 r = mul2(v.r2, invr);
+    const float2 rho_j = f2(d.z, d.w), s_j = f2(b.z, b.w);
+    float2 hi, hj, di = f2(0.0f), dj = f2(0.0f);
+    const Near2 late_i = hctSeries2<STORE, BRANCH>(r, invr, rho_i, s_j, &hi, &di);
+    const Near2 late_j = hctSeries2<STORE, BRANCH>(r, invr, rho_j, s_i, &hj, &dj);
+    const bool late_x = late_i.x || late_j.x;
+    const bool late_y = late_i.y || late_j.y;
     if (NECK) {
-      if (r.x < bi.w + bj1.w + neck.reach) {
-        const int nj = s.neck[js1];
-        hi.x += neck.integral(ni, nj, r.x);
-        hj.x += neck.integral(nj, ni, r.x);
+      if (!late_x && r.x < rho_i.x + rho_j.x + neck.reach) {
+        const int nj = s.neck[jneck + q];
+        float e, f;
+        hi.x += neck.both(ni, nj, r.x, invr.x, &e);
+        hj.x += neck.both(nj, ni, r.x, invr.x, &f);
+        di.x += e;
+        dj.x += f;
       }
-      if (r.y < bi.w + bj2.w + neck.reach) {
-        const int nj = s.neck[js2];
-        hi.y += neck.integral(ni, nj, r.y);
-        hj.y += neck.integral(nj, ni, r.y);
+      if (!late_y && r.y < rho_i.y + rho_j.y + neck.reach) {
+        const int nj = s.neck[jneck + q + 16];
+        float e, f;
+        hi.y += neck.both(ni, nj, r.y, invr.y, &e);
+        hj.y += neck.both(nj, ni, r.y, invr.y, &f);
+        di.y += e;
+        dj.y += f;
       }
     }
-    const float2 wneg = f2(-1.0f, -w2);
-    psi_i2 = fma2(hi, wneg, psi_i2);
-    psi_j = fma2(hj, wneg, psi_j);
+    late |= (late_x ? bit : 0u) | (late_y ? bit << 16 : 0u);
+    const float2 keep = f2(late_x ? 0.0f : (GUARD ? -wt.x : -1.0f),
+                           late_y ? 0.0f : (GUARD ? -wt.y : -1.0f));
+    psi_i = fma2(hi, keep, psi_i);
+    psi_j = fma2(hj, keep, psi_j);
+    if (STORE) {
+      __stcg(out, make_float4(di.x, di.y, dj.x, dj.y));
+    }
   }
-  __device__ __forceinline__ void rotate2(int lane) {
-    psi_j.x = __shfl_sync(kFullMask, psi_j.x, (lane + 1) & 31);
-    psi_j.y = __shfl_sync(kFullMask, psi_j.y, (lane + 1) & 31);
+  __device__ __forceinline__ void rotate(int src) {
+    psi_j.x = __shfl_sync(kFullMask, psi_j.x, src);
+    psi_j.y = __shfl_sync(kFullMask, psi_j.y, src);
+    bit <<= 1;
+    if (STORE) {
+      out += 32;
+    }
   }
-  __device__ __forceinline__ void merge(int src) {
-    psi_i = psi_i2.x + psi_i2.y;
-    psi_j1 = psi_j.x + __shfl_sync(kFullMask, psi_j.y, src);
+  // The pairs left out, after the walk; add(slot, v) adds v to a slot's descreening sum, and
+  // tile_out is the tile's first entry of the store
+  template <class Add>
+  __device__ __forceinline__ void finish(const TileInfo &ti, int lane, unsigned short* list,
+                                         float4* tile_out, const Add &add) const {
+    spreadLate(late, list, lane, [&](int of, int b) {
+      const LatePair p(s, ti, of, b);
+      const float4 c = hctClosed2<STORE>(p.r, p.r2, p.invr, p.rho, p.sj);
+      float2 h = f2(c.x, c.y), hd = f2(c.z, c.w);
+      if (NECK && p.r < p.rho.x + p.rho.y + neck.reach) {
+        const int a = s.neck[p.islot], z = s.neck[p.jslot];
+        float e, f;
+        h.x += neck.both(a, z, p.r, p.invr, &e);
+        h.y += neck.both(z, a, p.r, p.invr, &f);
+        hd.x += e;
+        hd.y += f;
+      }
+      add(p.islot, -h.x);
+      add(p.jslot, -h.y);
+      if (STORE) {
+        float* entry = reinterpret_cast<float*>(tile_out + 32 * p.step + of) + (b >> 4);
+        __stcg(entry, hd.x);
+        __stcg(entry + 2, hd.y);
+      }
+    });
   }
 };
 
 // Pass 2: Coulomb + Lennard-Jones on non-excluded pairs and the GB pair terms; with CLASH, the
 // Coulomb and Lennard-Jones terms of a molecule given a clash distance or ratio take softened
-// cores (the uniform branch is per tile: a tile belongs to one molecule)
+// cores (the uniform branch is per tile: a tile belongs to one molecule).  Energies are summed
+// negated (flush turns them), and both sides' forces as fmag x (r_j - r_i): block I's as they are,
+// block J's to be negated by the caller.
 template <bool FORCE, bool ENERGY, bool NB, bool GB, bool CLASH = false>
 struct PairPass {
+  static constexpr int kUnroll = 2;
   const UnitSmem &s;
   float kk, inv_diel;
   bool salt;
-  float4 ai, bi;
-  float inv4ri;     // 1 / (4 R_i)
+  AtomI at;
+  float2 q_i, r_i;  // charge and effective radius of atom i
+  float2 m4r_i;     // -1 / (4 R_i)
   int code_i;
   unsigned mask;
   bool soft;        // softened cores on this tile
   float clash_d, clash_r;
   float2 qcore;
-  float fxi, fyi, fzi, dei, fxj, fyj, fzj, dej;
-  float e_elec, e_vdw, e_gb;        // FP32 sums of at most eight pairs (see tileFlush)
+  float2 fxi, fyi, fzi, dei, fxj, fyj, fzj, dej;
+  float2 e_elec, e_vdw, e_gb;       // FP32 sums of at most eight pairs each (see tileFlush)
   double t_elec, t_vdw, t_gb;       // this lane's FP64 sums over the tile (see tileEnergy)
   __device__ PairPass(const UnitSmem &s_in, float kappa, float inv_dielectric) :
       s(s_in), kk(-kappa * kGbKscale), inv_diel(inv_dielectric), salt(kappa > 0.0f) {}
   __device__ __forceinline__ void flush() {
     if (ENERGY) {
-      t_elec += static_cast<double>(e_elec);
-      t_vdw += static_cast<double>(e_vdw);
-      t_gb += static_cast<double>(e_gb);
-      e_elec = e_vdw = e_gb = 0.0f;
+      if (NB) {
+        t_elec -= static_cast<double>(e_elec.x) + static_cast<double>(e_elec.y);
+        t_vdw -= static_cast<double>(e_vdw.x) + static_cast<double>(e_vdw.y);
+      }
+      if (GB) {
+        t_gb -= static_cast<double>(e_gb.x) + static_cast<double>(e_gb.y);
+      }
+      e_elec = e_vdw = e_gb = f2(0.0f);
     }
   }
-  __device__ __forceinline__ void begin(int islot, unsigned mask_in,
+  __device__ __forceinline__ void begin(const TileInfo &ti, const TileWalk &w, unsigned mask_in,
                                         float2 clash = make_float2(0.0f, 0.0f)) {
-    ai = s.pa[islot];
-    bi = s.pb[islot];
-    inv4ri = 0.25f * s.gbv[islot].x;
-    code_i = __float_as_int(s.prm[islot].y) & 0xffff;
+    const int islot = ti.ibase + w.il;
+    at.load(s, islot);
+    q_i = f2(slotValue(s.pb, islot, 2));
+    r_i = f2(slotValue(s.pd, islot, 2));
+    m4r_i = f2(-0.25f * slotValue(s.pg, islot, 0));
+    code_i = __float_as_int(slotValue(s.pg, islot, 2)) & 0xffff;
     mask = mask_in;
     if (CLASH) {
       clash_d = clash.x;
@@ -1121,101 +1315,125 @@ struct PairPass {
       soft = (clash.x > 0.0f || clash.y > 0.0f);
       qcore = quadraticCore(clash.x);
     }
-    fxi = fyi = fzi = dei = 0.0f;
-    fxj = fyj = fzj = dej = 0.0f;
-    e_elec = e_vdw = e_gb = 0.0f;
+    fxi = fyi = fzi = dei = f2(0.0f);
+    fxj = fyj = fzj = dej = f2(0.0f);
+    e_elec = e_vdw = e_gb = f2(0.0f);
     t_elec = t_vdw = t_gb = 0.0;
   }
-  __device__ __forceinline__ void pair(int jslot, int jl) {
-    const float4 aj = s.pa[jslot];
-    const float4 bj = s.pb[jslot];
-    const float2 gj = s.gbv[jslot];    // pass 2: 1 / effective radius, Lennard-Jones code bits
-    const float hx = aj.x - ai.x, hy = aj.y - ai.y, hz = aj.z - ai.z;
-    const float lx = bj.x - bi.x, ly = bj.y - bi.y, lz = bj.z - bi.z;
-    const float3 dv = make_float3(hx + lx, hy + ly, hz + lz);
-    const float r2 = fmaf(dv.x, dv.x, fmaf(dv.y, dv.y, dv.z * dv.z));
-    const float qiqj_all = ai.w * aj.w;
-    float fmag = 0.0f;
+  template <bool GUARD>
+  __device__ __forceinline__ void pair(int rec, int q, float2 wt) {
+    const float4 a = s.pa[rec], b = s.pb[rec], c = s.pc[rec], d = s.pd[rec], g = s.pg[rec];
+    const Separation2 v = separate2<GUARD>(at, a, b, c, d, wt);
+    const float2 r2 = v.r2;
+    float2 qq = mul2(q_i, f2(b.z, b.w));
+    if (GUARD) {
+      qq = mul2(qq, wt);
+    }
+    float2 fmag = f2(0.0f);
     if (NB) {
-      // excluded and padding pairs take the same path with zero parameters
-      const float incl = ((mask >> jl) & 1u) ? 0.0f : 1.0f;
+      // excluded and padding pairs take the same path with zero parameters; nincl is -1 or 0
+      const unsigned m = mask >> q;
+      float2 nincl = f2((m & 1u) ? 0.0f : -1.0f, (m & 0x10000u) ? 0.0f : -1.0f);
+      if (GUARD) {
+        nincl = mul2(nincl, wt);
+      }
       // 1/r from rsqrt with one Newton step (Coulomb), and 1/r^2 as its own reciprocal: r^-6
       // and r^-12 multiply the relative error of 1/r^2 by 3 and 6, so squaring 1/r (twice its
       // error) would double the rounding of the repulsive wall, and the Newton step of 1/r^2
       // takes the exact r^2 = r2 + 2 (dx ex + dy ey + dz ez) + O(e^2), the e the separations'
-      // recovered rounding errors (separationError): without it the Lennard-Jones energy of a
+      // recovered rounding errors (splitCoordinate): without it the Lennard-Jones energy of a
       // molecule with close contacts errs by up to 1.5e-6 of the root-sum-square of its pair
       // terms.  r2 >= 256 on padding slots, never zero.
-      float invr = rsqrtf(r2);
-      invr = invr * fmaf(-0.5f * r2 * invr, invr, 1.5f);
-      const float r2c = fmaf(dv.x, separationError(hx, lx, dv.x),
-                             fmaf(dv.y, separationError(hy, ly, dv.y),
-                                  dv.z * separationError(hz, lz, dv.z)));
-      float invr2 = __fdividef(1.0f, r2);
-      invr2 = fmaf(invr2, fmaf(-2.0f * r2c, invr2, fmaf(-r2, invr2, 1.0f)), invr2);
-      const float invr6 = invr2 * invr2 * invr2;
-      float2 ab = s.lj[code_i + (__float_as_int(gj.y) >> 16)];
-      ab.x *= incl;
-      ab.y *= incl;
-      const float qiqj = qiqj_all * incl;
+      float2 invr = f2(rsqrtf(r2.x), rsqrtf(r2.y));
+      invr = mul2(invr, fma2(mul2(mul2(r2, f2(-0.5f)), invr), invr, f2(1.5f)));
+      const float2 ex = sub2(v.lx, sub2(v.dx, v.hx));
+      const float2 ey = sub2(v.ly, sub2(v.dy, v.hy));
+      const float2 ez = sub2(v.lz, sub2(v.dz, v.hz));
+      float2 m2r2c = fma2(v.dx, ex, fma2(v.dy, ey, mul2(v.dz, ez)));
+      m2r2c = mul2(m2r2c, f2(-2.0f));
+      float2 invr2 = f2(__fdividef(1.0f, r2.x), __fdividef(1.0f, r2.y));
+      const float2 step = fma2(m2r2c, invr2, fma2(mul2(r2, f2(-1.0f)), invr2, f2(1.0f)));
+      invr2 = fma2(invr2, step, invr2);
+      const float2 invr6 = mul2(mul2(invr2, invr2), invr2);
+      const float2 ab1 = s.lj[code_i + (__float_as_int(g.z) >> 16)];
+      const float2 ab2 = s.lj[code_i + (__float_as_int(g.w) >> 16)];
+      const float2 nqq = mul2(qq, nincl);
+      const float2 nla = mul2(f2(ab1.x, ab2.x), nincl);
+      const float2 nlb = mul2(f2(ab1.y, ab2.y), nincl);
       if (CLASH && soft) {
-        fmag = softCorePair(r2 * invr, invr, qiqj, ab.x, ab.y, clash_d, qcore, clash_r, &e_elec,
-                            &e_vdw);
+        float ee = 0.0f, ev = 0.0f;
+        fmag.x = softCorePair(r2.x * invr.x, invr.x, -nqq.x, -nla.x, -nlb.x, clash_d, qcore,
+                              clash_r, &ee, &ev);
+        e_elec.x -= ee;
+        e_vdw.x -= ev;
+        ee = ev = 0.0f;
+        fmag.y = softCorePair(r2.y * invr.y, invr.y, -nqq.y, -nla.y, -nlb.y, clash_d, qcore,
+                              clash_r, &ee, &ev);
+        e_elec.y -= ee;
+        e_vdw.y -= ev;
       }
       else {
+        // -(A / r^6 - B)
+        const float2 nw = fma2(nla, invr6, mul2(nlb, f2(-1.0f)));
         if (ENERGY) {
-          e_elec = __fadd_rn(e_elec, __fmul_rn(qiqj, invr));
-          e_vdw = __fadd_rn(e_vdw, __fmul_rn(__fsub_rn(__fmul_rn(ab.x, invr6), ab.y), invr6));
+          e_elec = fma2(nqq, invr, e_elec);                       // minus the energy
+          e_vdw = fma2(nw, invr6, e_vdw);
         }
         if (FORCE) {
-          fmag = -(qiqj * invr * invr2) + (6.0f * ab.y - 12.0f * ab.x * invr6) * invr6 * invr2;
+          // -(qq / r^3) + (6 B - 12 A / r^6) / r^8
+          fmag = mul2(invr2, fma2(nqq, invr, mul2(mul2(invr6, f2(6.0f)), fma2(nla, invr6, nw))));
         }
       }
     }
     if (GB) {
-      const float qiqj = qiqj_all;
-      const float ijb = bi.w * bj.w;
-      const float efac = __expf(-r2 * inv4ri * gj.x);
-      const float fgbi = rsqrtf(fmaf(ijb, efac, r2));
-      float expmkf, fgbk;
+      const float2 ijb = mul2(r_i, f2(d.z, d.w));
+      const float2 arg = mul2(mul2(r2, m4r_i), f2(g.x, g.y));
+      const float2 efac = f2(__expf(arg.x), __expf(arg.y));
+      const float2 f2gb = fma2(ijb, efac, r2);
+      const float2 fgbi = f2(rsqrtf(f2gb.x), rsqrtf(f2gb.y));
+      float2 dielfac, chain;       // 1 - exp(...) / diel, and the same plus its r derivative's part
       if (salt) {
-        fgbk = __fdividef(kk, fgbi);
-        expmkf = __expf(fgbk) * inv_diel;
+        const float2 fgbk = f2(__fdividef(kk, fgbi.x), __fdividef(kk, fgbi.y));
+        const float2 expmkf = f2(__expf(fgbk.x) * inv_diel, __expf(fgbk.y) * inv_diel);
+        dielfac = f2(1.0f - expmkf.x, 1.0f - expmkf.y);
+        chain = fma2(fgbk, expmkf, dielfac);
       }
       else {
-        fgbk = 0.0f;
-        expmkf = inv_diel;
+        dielfac = f2(1.0f - inv_diel);
+        chain = dielfac;
       }
-      const float dielfac = 1.0f - expmkf;
+      const float2 qf = mul2(qq, fgbi);
       if (ENERGY) {
-        e_gb = __fsub_rn(e_gb, __fmul_rn(__fmul_rn(qiqj, dielfac), fgbi));
+        e_gb = fma2(qf, dielfac, e_gb);                           // minus the energy
       }
       if (FORCE) {
-        const float temp4 = fgbi * fgbi * fgbi;
-        const float temp6 = qiqj * temp4 * fmaf(fgbk, expmkf, dielfac);
-        fmag += temp6 * fmaf(-0.25f, efac, 1.0f);
-        const float temp5 = 0.5f * efac * temp6 * fmaf(0.25f, r2, ijb);
-        dei = fmaf(bi.w, temp5, dei);
-        dej = fmaf(bj.w, temp5, dej);
+        const float2 temp6 = mul2(mul2(qf, mul2(fgbi, fgbi)), chain);
+        fmag = fma2(temp6, fma2(f2(-0.25f), efac, f2(1.0f)), fmag);
+        const float2 temp5 = mul2(mul2(mul2(efac, f2(0.5f)), temp6), fma2(f2(0.25f), r2, ijb));
+        dei = fma2(r_i, temp5, dei);
+        dej = fma2(f2(d.z, d.w), temp5, dej);
       }
     }
     if (FORCE) {
-      fxi = fmaf(fmag, dv.x, fxi);
-      fyi = fmaf(fmag, dv.y, fyi);
-      fzi = fmaf(fmag, dv.z, fzi);
-      fxj = fmaf(-fmag, dv.x, fxj);
-      fyj = fmaf(-fmag, dv.y, fyj);
-      fzj = fmaf(-fmag, dv.z, fzj);
+      fxi = fma2(fmag, v.dx, fxi);
+      fyi = fma2(fmag, v.dy, fyi);
+      fzi = fma2(fmag, v.dz, fzi);
+      fxj = fma2(fmag, v.dx, fxj);
+      fyj = fma2(fmag, v.dy, fyj);
+      fzj = fma2(fmag, v.dz, fzj);
     }
   }
-  __device__ __forceinline__ void rotate(int lane) {
+  __device__ __forceinline__ void rotate(int src) {
     if (FORCE) {
-      const int src = (lane + 1) & 31;
-      fxj = __shfl_sync(kFullMask, fxj, src);
-      fyj = __shfl_sync(kFullMask, fyj, src);
-      fzj = __shfl_sync(kFullMask, fzj, src);
+      fxj.x = __shfl_sync(kFullMask, fxj.x, src);
+      fxj.y = __shfl_sync(kFullMask, fxj.y, src);
+      fyj.x = __shfl_sync(kFullMask, fyj.x, src);
+      fyj.y = __shfl_sync(kFullMask, fyj.y, src);
+      fzj.x = __shfl_sync(kFullMask, fzj.x, src);
+      fzj.y = __shfl_sync(kFullMask, fzj.y, src);
       if (GB) {
-        dej = __shfl_sync(kFullMask, dej, src);
+        dej.x = __shfl_sync(kFullMask, dej.x, src);
+        dej.y = __shfl_sync(kFullMask, dej.y, src);
       }
     }
   }
@@ -1226,155 +1444,152 @@ __device__ __forceinline__ void tileFlush(PairPass<FORCE, ENERGY, NB, GB, CLASH>
   p.flush();
 }
 
-// Pass 3: radius chain-rule forces
+// Pass 3 of the tiled path: radius chain-rule forces, the HCT derivatives evaluated again (the
+// pair-derivative store would cost more bytes there than the arithmetic it saves)
 template <bool NECK = false>
 struct DerivPass {
+  static constexpr int kUnroll = 2;
   const UnitSmem &s;
   NeckGb neck;
-  float4 ai, bi;
-  int ni;
-  float de_i;
-  float fxi, fyi, fzi, fxj, fyj, fzj;
+  AtomI at;
+  float2 rho_i, s_i, de_i;
+  int ni, jneck;
+  unsigned late, bit;
+  float2 fxi, fyi, fzi, fxj, fyj, fzj;
   __device__ DerivPass(const UnitSmem &s_in, const DevSynthesis &d) : s(s_in), neck(d) {}
-  __device__ __forceinline__ void begin(int islot) {
-    ai = s.pa[islot];
-    bi = s.pb[islot];
+  __device__ __forceinline__ void begin(const TileInfo &ti, const TileWalk &w) {
+    const int islot = ti.ibase + w.il;
+    at.load(s, islot);
+    rho_i = f2(slotValue(s.pd, islot, 2));
+    s_i = f2(slotValue(s.pb, islot, 2));
+    de_i = f2(slotValue(s.pg, islot, 2));
     if (NECK) {
       ni = s.neck[islot];
+      jneck = ti.jbase;
     }
-    de_i = s.gbv[islot].y;
-    fxi = fyi = fzi = 0.0f;
-    fxj = fyj = fzj = 0.0f;
+    late = 0u;
+    bit = 1u;
+    fxi = fyi = fzi = f2(0.0f);
+    fxj = fyj = fzj = f2(0.0f);
   }
-  __device__ __forceinline__ void pair(int jslot, int) {
-    const float4 aj = s.pa[jslot];
-    const float4 bj = s.pb[jslot];
-    const float de_j = s.gbv[jslot].y;
-    const float3 dv = pairDelta(ai, bi, aj, bj);
-    const float r2 = fmaf(dv.x, dv.x, fmaf(dv.y, dv.y, dv.z * dv.z));
-    const float invr = rsqrtf(r2);
-    const float r = r2 * invr;
-    // scalar forms: on the long chains of the tiled path nearly every pair is far, and the
-    // packed pair form measured slower there
-    float fmag = hctDerivative(r, r2, invr, bi.w, aj.w) * de_i +
-                 hctDerivative(r, r2, invr, bj.w, ai.w) * de_j;
-    if (NECK && r < bi.w + bj.w + neck.reach) {
-      const int nj = s.neck[jslot];
-      float dij, dji;
-      neck.both(ni, nj, r, invr, &dij);
-      neck.both(nj, ni, r, invr, &dji);
-      fmag += dij * de_i + dji * de_j;
-    }
-    fxi = fmaf(-fmag, dv.x, fxi);
-    fyi = fmaf(-fmag, dv.y, fyi);
-    fzi = fmaf(-fmag, dv.z, fzi);
-    fxj = fmaf(fmag, dv.x, fxj);
-    fyj = fmaf(fmag, dv.y, fyj);
-    fzj = fmaf(fmag, dv.z, fzj);
+  __device__ __forceinline__ float neckForce(int a, int z, float r, float invr, float de_a,
+                                             float de_z) const {
+    float da, dz;
+    neck.both(a, z, r, invr, &da);
+    neck.both(z, a, r, invr, &dz);
+    return da * de_a + dz * de_z;
   }
-  __device__ __forceinline__ void rotate(int lane) {
-    const int src = (lane + 1) & 31;
-    fxj = __shfl_sync(kFullMask, fxj, src);
-    fyj = __shfl_sync(kFullMask, fyj, src);
-    fzj = __shfl_sync(kFullMask, fzj, src);
-  }
-};
-
-// GB pass 1 of a force evaluation: psi_i -= H(r, rho_i, s_j rho_j), psi_j -= H(r, rho_j,
-// s_i rho_i), and the radial derivatives of both terms stored for pass 3 (one float2 per lane
-// and step of the tile walk, so the stores of a step are one coalesced 256-byte line)
-template <bool NECK = false>
-struct RadiiDerivPass {
-  const UnitSmem &s;
-  NeckGb neck;
-  float4 ai, bi;
-  int ni;
-  float psi_i, psi_j;   // i-side sum, traveling j-side sum
-  float2* out;          // this lane's entry for the current step
-  __device__ RadiiDerivPass(const UnitSmem &s_in, const DevSynthesis &d) : s(s_in), neck(d) {}
-  __device__ __forceinline__ void begin(int islot, float2* tile_out) {
-    ai = s.pa[islot];
-    bi = s.pb[islot];
+  template <bool GUARD>
+  __device__ __forceinline__ void pair(int rec, int q, float2 wt) {
+    const float4 a = s.pa[rec], b = s.pb[rec], c = s.pc[rec], d = s.pd[rec], g = s.pg[rec];
+    const Separation2 v = separate2<GUARD>(at, a, b, c, d, wt);
+    const float2 invr = f2(rsqrtf(v.r2.x), rsqrtf(v.r2.y));
+    const float2 r = mul2(v.r2, invr);
+    const float2 rho_j = f2(d.z, d.w), s_j = f2(b.z, b.w), de_j = f2(g.z, g.w);
+    float2 unused, di, dj;
+    const Near2 late_i = hctSeries2<true, true>(r, invr, rho_i, s_j, &unused, &di);
+    const Near2 late_j = hctSeries2<true, true>(r, invr, rho_j, s_i, &unused, &dj);
+    const bool late_x = late_i.x || late_j.x;
+    const bool late_y = late_i.y || late_j.y;
+    float2 fmag = fma2(di, de_i, mul2(dj, de_j));
     if (NECK) {
-      ni = s.neck[islot];
+      if (!late_x && r.x < rho_i.x + rho_j.x + neck.reach) {
+        fmag.x += neckForce(ni, s.neck[jneck + q], r.x, invr.x, de_i.x, de_j.x);
+      }
+      if (!late_y && r.y < rho_i.y + rho_j.y + neck.reach) {
+        fmag.y += neckForce(ni, s.neck[jneck + q + 16], r.y, invr.y, de_i.y, de_j.y);
+      }
     }
-    psi_i = 0.0f;
-    psi_j = 0.0f;
-    out = tile_out;
-  }
-  __device__ __forceinline__ void pair(int jslot, int) {
-    const float4 aj = s.pa[jslot];
-    const float4 bj = s.pb[jslot];
-    const float2 dxy = add2(sub2(f2(aj.x, aj.y), f2(ai.x, ai.y)),
-                            sub2(f2(bj.x, bj.y), f2(bi.x, bi.y)));
-    const float dz = (aj.z - ai.z) + (bj.z - bi.z);
-    const float r2 = fmaf(dxy.x, dxy.x, fmaf(dxy.y, dxy.y, dz * dz));
-    const float invr = rsqrtf(r2);
-    const float r = r2 * invr;
-    float2 h, hd;
-    hctBoth2(r, r2, invr, f2(bi.w, bj.w), f2(aj.w, ai.w), &h, &hd);
-    if (NECK && r < bi.w + bj.w + neck.reach) {
-      const int nj = s.neck[jslot];
-      float dij, dji;
-      h.x += neck.both(ni, nj, r, invr, &dij);
-      h.y += neck.both(nj, ni, r, invr, &dji);
-      hd.x += dij;
-      hd.y += dji;
+    late |= (late_x ? bit : 0u) | (late_y ? bit << 16 : 0u);
+    if (GUARD) {
+      fmag = mul2(fmag, wt);
     }
-    psi_i -= h.x;
-    psi_j -= h.y;
-    __stcg(out, hd);
+    fmag = f2(late_x ? 0.0f : fmag.x, late_y ? 0.0f : fmag.y);
+    fxi = fma2(fmag, v.dx, fxi);
+    fyi = fma2(fmag, v.dy, fyi);
+    fzi = fma2(fmag, v.dz, fzi);
+    fxj = fma2(fmag, v.dx, fxj);
+    fyj = fma2(fmag, v.dy, fyj);
+    fzj = fma2(fmag, v.dz, fzj);
   }
-  __device__ __forceinline__ void rotate(int lane) {
-    psi_j = __shfl_sync(kFullMask, psi_j, (lane + 1) & 31);
-    out += 32;
+  __device__ __forceinline__ void rotate(int src) {
+    fxj.x = __shfl_sync(kFullMask, fxj.x, src);
+    fxj.y = __shfl_sync(kFullMask, fxj.y, src);
+    fyj.x = __shfl_sync(kFullMask, fyj.x, src);
+    fyj.y = __shfl_sync(kFullMask, fyj.y, src);
+    fzj.x = __shfl_sync(kFullMask, fzj.x, src);
+    fzj.y = __shfl_sync(kFullMask, fzj.y, src);
+    bit <<= 1;
+  }
+  // The pairs hctSeries2 left out, after the walk; add(slot, fx, fy, fz) adds to a slot's force
+  template <class Add>
+  __device__ __forceinline__ void finish(const TileInfo &ti, int lane, unsigned short* list,
+                                         const Add &add) const {
+    spreadLate(late, list, lane, [&](int of, int b) {
+      const LatePair p(s, ti, of, b);
+      const float4 c = hctClosed2<true>(p.r, p.r2, p.invr, p.rho, p.sj);
+      const float de_a = slotValue(s.pg, p.islot, 2), de_z = slotValue(s.pg, p.jslot, 2);
+      float fmag = fmaf(c.z, de_a, c.w * de_z);
+      if (NECK && p.r < p.rho.x + p.rho.y + neck.reach) {
+        fmag += neckForce(s.neck[p.islot], s.neck[p.jslot], p.r, p.invr, de_a, de_z);
+      }
+      add(p.islot, -fmag * p.dv.x, -fmag * p.dv.y, -fmag * p.dv.z);
+      add(p.jslot, fmag * p.dv.x, fmag * p.dv.y, fmag * p.dv.z);
+    });
   }
 };
 
 // Pass 3 from the stored derivatives: the force of a pair is (hd_i dE/dR_i + hd_j dE/dR_j) times
-// the separation, with no transcendental left to evaluate
+// the separation, with no transcendental left to evaluate.  Both sides sum +force x separation;
+// the caller negates block I's.
 struct DerivStoredPass {
+  static constexpr int kUnroll = 4;
   const UnitSmem &s;
-  float4 ai, bi;
-  float de_i;
-  float2 fxyi, fxyj;
-  float fzi, fzj;
-  const float2* in;
+  AtomI at;
+  float2 de_i;
+  float2 fxi, fyi, fzi, fxj, fyj, fzj;
+  const float4* in;
   __device__ DerivStoredPass(const UnitSmem &s_in) : s(s_in) {}
-  __device__ __forceinline__ void begin(int islot, const float2* tile_in) {
-    ai = s.pa[islot];
-    bi = s.pb[islot];
-    de_i = s.gbv[islot].y;
-    fxyi = fxyj = f2(0.0f);
-    fzi = fzj = 0.0f;
+  __device__ __forceinline__ void begin(const TileInfo &ti, const TileWalk &w,
+                                        const float4* tile_in) {
+    const int islot = ti.ibase + w.il;
+    at.load(s, islot);
+    de_i = f2(slotValue(s.pg, islot, 2));
+    fxi = fyi = fzi = f2(0.0f);
+    fxj = fyj = fzj = f2(0.0f);
     in = tile_in;
   }
-  __device__ __forceinline__ void pair(int jslot, int) {
-    const float2 hd = __ldcs(in);
-    const float4 aj = s.pa[jslot];
-    const float4 bj = s.pb[jslot];
-    const float de_j = s.gbv[jslot].y;
-    const float2 dxy = add2(sub2(f2(aj.x, aj.y), f2(ai.x, ai.y)),
-                            sub2(f2(bj.x, bj.y), f2(bi.x, bi.y)));
-    const float dz = (aj.z - ai.z) + (bj.z - bi.z);
-    const float fmag = fmaf(hd.y, de_j, hd.x * de_i);
-    fxyi = fma2(f2(-fmag), dxy, fxyi);
-    fzi = fmaf(-fmag, dz, fzi);
-    fxyj = fma2(f2(fmag), dxy, fxyj);
-    fzj = fmaf(fmag, dz, fzj);
+  template <bool GUARD>
+  __device__ __forceinline__ void pair(int rec, int, float2 wt) {
+    const float4 hd = __ldcs(in);
+    const float4 a = s.pa[rec], b = s.pb[rec], c = s.pc[rec], d = s.pd[rec], g = s.pg[rec];
+    const Separation2 v = separate2<false>(at, a, b, c, d, wt);
+    float2 fmag = fma2(f2(hd.x, hd.y), de_i, mul2(f2(hd.z, hd.w), f2(g.z, g.w)));
+    if (GUARD) {
+      fmag = f2(wt.x != 0.0f ? fmag.x : 0.0f, wt.y != 0.0f ? fmag.y : 0.0f);
+    }
+    fxi = fma2(fmag, v.dx, fxi);
+    fyi = fma2(fmag, v.dy, fyi);
+    fzi = fma2(fmag, v.dz, fzi);
+    fxj = fma2(fmag, v.dx, fxj);
+    fyj = fma2(fmag, v.dy, fyj);
+    fzj = fma2(fmag, v.dz, fzj);
   }
-  __device__ __forceinline__ void rotate(int lane) {
-    const int src = (lane + 1) & 31;
-    fxyj.x = __shfl_sync(kFullMask, fxyj.x, src);
-    fxyj.y = __shfl_sync(kFullMask, fxyj.y, src);
-    fzj = __shfl_sync(kFullMask, fzj, src);
+  __device__ __forceinline__ void rotate(int src) {
+    fxj.x = __shfl_sync(kFullMask, fxj.x, src);
+    fxj.y = __shfl_sync(kFullMask, fxj.y, src);
+    fyj.x = __shfl_sync(kFullMask, fyj.x, src);
+    fyj.y = __shfl_sync(kFullMask, fyj.y, src);
+    fzj.x = __shfl_sync(kFullMask, fzj.x, src);
+    fzj.y = __shfl_sync(kFullMask, fzj.y, src);
     in += 32;
   }
 };
 
-// Entry of lane 0, step 0 of tile t of a unit whose tiles start at tile_base in the store
-__device__ __forceinline__ size_t pairDerivOffset(int tile_base, int t) {
-  return static_cast<size_t>(tile_base + t) * kPairDerivPerTile;
+// This lane's entry for step 0 of tile t of a unit whose tiles start at tile_base in the store
+__device__ __forceinline__ float4* pairDerivTile(const DevSynthesis &d, int tile_base, int t,
+                                                 int lane) {
+  return d.pair_deriv + static_cast<size_t>(tile_base + t) * kPairDerivPerTile + lane;
 }
 
 template <bool STORE, bool NECK>
@@ -1382,34 +1597,27 @@ __device__ void gbRadiiTiles(const DevSynthesis &d, const UnitSmem &s, int nsys_
                              int tile_base, int first, int stride) {
   const int lane = threadIdx.x & 31;
   const float ps = static_cast<float>(1 << kPsiBits);
-  if (STORE) {
-    RadiiDerivPass<NECK> p(s, d);
-    for (int t = first; t < ntiles; t += stride) {
-      const TileInfo ti = tileInfo(s, nsys_u, t);
-      p.begin(ti.ibase + lane, d.pair_deriv + pairDerivOffset(tile_base, t) + lane);
-      walkTile(p, ti, lane);
-      if (lane < ti.ni) {
-        atomicAddInt63(p.psi_i * ps, &s.psi[ti.ibase + lane], &s.psio[ti.ibase + lane]);
-      }
-      const int jl = traveledAtom(ti, lane);
-      if (jl < ti.nj) {
-        atomicAddInt63(p.psi_j * ps, &s.psi[ti.jbase + jl], &s.psio[ti.jbase + jl]);
-      }
-    }
-    return;
-  }
-  RadiiPass2<NECK> p(s, d);
+  unsigned short* list = s.late + (threadIdx.x >> 5) * kLateEntries;
+  const auto add = [&](int slot, float v) {
+    atomicAddInt63(v * ps, &s.psi[slot], &s.psio[slot]);
+  };
+  RadiiPass<STORE, NECK> p(s, d);
   for (int t = first; t < ntiles; t += stride) {
     const TileInfo ti = tileInfo(s, nsys_u, t);
-    p.begin(ti.ibase + lane);
-    walkTile2(p, ti, lane);
-    if (lane < ti.ni) {
-      atomicAddInt63(p.psi_i * ps, &s.psi[ti.ibase + lane], &s.psio[ti.ibase + lane]);
+    const TileWalk w = tileWalk(ti, lane);
+    float4* out = STORE ? pairDerivTile(d, tile_base, t, lane) : nullptr;
+    p.begin(ti, w, out);
+    walkTile(p, ti, w, lane);
+    const float vi = iShare(p.psi_i, w);
+    const float vj = jShare(p.psi_j, w, lane);
+    if (ownsAtom(ti, w, lane)) {
+      add(ti.ibase + lane, vi);
     }
-    const int jl = traveledAtom2(ti, lane);
+    const int jl = sharedAtom(w, lane);
     if (jl < ti.nj) {
-      atomicAddInt63(p.psi_j1 * ps, &s.psi[ti.jbase + jl], &s.psio[ti.jbase + jl]);
+      add(ti.jbase + jl, vj);
     }
+    p.finish(ti, lane, list, STORE ? out - lane : nullptr, add);
   }
 }
 
@@ -1439,6 +1647,7 @@ __device__ void pairTiles(const DevSynthesis &d, const UnitSmem &s, int nsys_u, 
   };
   for (int t = first; t < ntiles; t += stride) {
     const TileInfo ti = tileInfo(s, nsys_u, t);
+    const TileWalk w = tileWalk(ti, lane);
     if (ENERGY && ti.k != acc_k) {
       commit();
       acc_k = ti.k;
@@ -1447,25 +1656,30 @@ __device__ void pairTiles(const DevSynthesis &d, const UnitSmem &s, int nsys_u, 
     if (NB) {
       const int midx = d.tile_mask_idx[d.tile_start[s.sys[ti.k]] + ti.local];
       if (midx != 0) {
-        mask = __ldg(&d.mask_pool[static_cast<size_t>(midx) * 32 + lane]);
+        mask = __ldg(&d.mask_pool[static_cast<size_t>(midx) * 32 + w.il]);
       }
     }
-    p.begin(ti.ibase + lane, mask, CLASH ? s.clash[ti.k] : make_float2(0.0f, 0.0f));
-    walkTile(p, ti, lane);
+    p.begin(ti, w, mask, CLASH ? s.clash[ti.k] : make_float2(0.0f, 0.0f));
+    walkTile(p, ti, w, lane);
     if (FORCE) {
-      if (lane < ti.ni) {
+      const float fxi = iShare(p.fxi, w), fyi = iShare(p.fyi, w), fzi = iShare(p.fzi, w);
+      const float dei = GB ? iShare(p.dei, w) : 0.0f;
+      const float fxj = jShare(p.fxj, w, lane), fyj = jShare(p.fyj, w, lane);
+      const float fzj = jShare(p.fzj, w, lane);
+      const float dej = GB ? jShare(p.dej, w, lane) : 0.0f;
+      if (ownsAtom(ti, w, lane)) {
         const int is = ti.ibase + lane;
-        addForce(s, is, p.fxi, p.fyi, p.fzi, fs);
+        addForce(s, is, fxi, fyi, fzi, fs);
         if (GB) {
-          atomicAddInt63(p.dei * ds, &s.de[is], &s.deo[is]);
+          atomicAddInt63(dei * ds, &s.de[is], &s.deo[is]);
         }
       }
-      const int jl = traveledAtom(ti, lane);
+      const int jl = sharedAtom(w, lane);
       if (jl < ti.nj) {
         const int js = ti.jbase + jl;
-        addForce(s, js, p.fxj, p.fyj, p.fzj, fs);
+        addForce(s, js, -fxj, -fyj, -fzj, fs);
         if (GB) {
-          atomicAddInt63(p.dej * ds, &s.de[js], &s.deo[js]);
+          atomicAddInt63(dej * ds, &s.de[js], &s.deo[js]);
         }
       }
     }
@@ -1491,14 +1705,18 @@ __device__ void gbDerivativeTiles(const DevSynthesis &d, const UnitSmem &s, int 
   DerivStoredPass p(s);
   for (int t = first; t < ntiles; t += stride) {
     const TileInfo ti = tileInfo(s, nsys_u, t);
-    p.begin(ti.ibase + lane, d.pair_deriv + pairDerivOffset(tile_base, t) + lane);
-    walkTile(p, ti, lane);
-    if (lane < ti.ni) {
-      addForce(s, ti.ibase + lane, p.fxyi.x, p.fxyi.y, p.fzi, fs);
+    const TileWalk w = tileWalk(ti, lane);
+    p.begin(ti, w, pairDerivTile(d, tile_base, t, lane));
+    walkTile(p, ti, w, lane);
+    const float fxi = iShare(p.fxi, w), fyi = iShare(p.fyi, w), fzi = iShare(p.fzi, w);
+    const float fxj = jShare(p.fxj, w, lane), fyj = jShare(p.fyj, w, lane);
+    const float fzj = jShare(p.fzj, w, lane);
+    if (ownsAtom(ti, w, lane)) {
+      addForce(s, ti.ibase + lane, -fxi, -fyi, -fzi, fs);
     }
-    const int jl = traveledAtom(ti, lane);
+    const int jl = sharedAtom(w, lane);
     if (jl < ti.nj) {
-      addForce(s, ti.jbase + jl, p.fxyj.x, p.fxyj.y, p.fzj, fs);
+      addForce(s, ti.jbase + jl, fxj, fyj, fzj, fs);
     }
   }
 }
@@ -1636,26 +1854,35 @@ __device__ __forceinline__ int slotNeck(const DevSynthesis &d, const UnitSmem &s
   return (d.neck_size > 0 && a < s.natom[k]) ? d.neck_idx[d.atom_start[s.sys[k]] + a] : 0;
 }
 
+// Write a slot's coordinates, payloads and GB values
+__device__ __forceinline__ void putSlot(const UnitSmem &s, int slot, float3 hi, float3 lo, float w1,
+                                        float w2, float g, float h) {
+  slotValue(s.pa, slot, 0) = hi.x;
+  slotValue(s.pa, slot, 2) = hi.y;
+  slotValue(s.pb, slot, 0) = hi.z;
+  slotValue(s.pb, slot, 2) = w1;
+  slotValue(s.pc, slot, 0) = lo.x;
+  slotValue(s.pc, slot, 2) = lo.y;
+  slotValue(s.pd, slot, 0) = lo.z;
+  slotValue(s.pd, slot, 2) = w2;
+  slotValue(s.pg, slot, 0) = g;
+  slotValue(s.pg, slot, 2) = h;
+}
+
 // Place an atom (fixed-point coordinates c, real = true) or a padding slot (far from everything:
 // 16 A apart along x beyond 5000 A) and clear its accumulators for a new evaluation
 __device__ __forceinline__ void placeSlot(const DevSynthesis &d, const UnitSmem &s, int slot,
                                           bool real, long long cx, long long cy, long long cz) {
   const float4 prm = s.prm[slot];
-  float4 pa, pb;
+  float3 hi = make_float3(5000.0f + 16.0f * static_cast<float>(slot), 0.0f, 0.0f);
+  float3 lo = make_float3(0.0f, 0.0f, 0.0f);
   if (real) {
-    splitCoordinate(static_cast<double>(cx) * d.inv_gpos_scale, &pa.x, &pb.x);
-    splitCoordinate(static_cast<double>(cy) * d.inv_gpos_scale, &pa.y, &pb.y);
-    splitCoordinate(static_cast<double>(cz) * d.inv_gpos_scale, &pa.z, &pb.z);
+    splitCoordinate(static_cast<double>(cx) * d.inv_gpos_scale, &hi.x, &lo.x);
+    splitCoordinate(static_cast<double>(cy) * d.inv_gpos_scale, &hi.y, &lo.y);
+    splitCoordinate(static_cast<double>(cz) * d.inv_gpos_scale, &hi.z, &lo.z);
   }
-  else {
-    pa = make_float4(5000.0f + 16.0f * static_cast<float>(slot), 0.0f, 0.0f, 0.0f);
-    pb = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  }
-  pa.w = prm.w;   // pass 1 payload: s * rho
-  pb.w = prm.z;   //                 rho
-  s.pa[slot] = pa;
-  s.pb[slot] = pb;
-  s.gbv[slot] = make_float2(1.0f, 0.0f);
+  // pass 1 payload: s * rho and rho
+  putSlot(s, slot, hi, lo, prm.w, prm.z, 1.0f, 0.0f);
   s.fx[slot] = 0;
   s.fy[slot] = 0;
   s.fz[slot] = 0;
@@ -1704,8 +1931,6 @@ __device__ void evaluateStaged(const DevSynthesis &d, const UnitSmem &s, const U
       const int k = findOwner(s.slot0, nsys_u, slot);
       const int a = slot - s.slot0[k];
       float e_self = 0.0f;
-      float4 pa = s.pa[slot];
-      float4 pb = s.pb[slot];
       const float4 prm = s.prm[slot];
       float egbi = 1.0f;
       if (a < s.natom[k]) {
@@ -1723,17 +1948,13 @@ __device__ void evaluateStaged(const DevSynthesis &d, const UnitSmem &s, const U
           d.psi[gi] = __double2ll_rn(static_cast<double>(psi) * d.psi_out_scale);
           d.psi_ovrf[gi] = 0;
         }
-        pa.w = prm.x;   // pass 2 payload: charge
-        pb.w = egbi;    //                 effective radius
       }
-      else {
-        pa.w = 0.0f;
-        pb.w = 1.0f;
-      }
-      s.pa[slot] = pa;
-      s.pb[slot] = pb;
-      // pass 2 reads a partner's reciprocal radius and Lennard-Jones code with one load
-      s.gbv[slot] = make_float2(1.0f / egbi, prm.y);
+      // pass 2 payload: charge (zero for padding, as prm.x is) and effective radius, and the
+      // reciprocal radius beside the Lennard-Jones code
+      slotValue(s.pb, slot, 2) = prm.x;
+      slotValue(s.pd, slot, 2) = egbi;
+      slotValue(s.pg, slot, 0) = 1.0f / egbi;
+      slotValue(s.pg, slot, 2) = prm.y;
       if (ENERGY) {
         warpEnergy(s, k, kGb, e_self, d.nrg_scale);
       }
@@ -1743,11 +1964,9 @@ __device__ void evaluateStaged(const DevSynthesis &d, const UnitSmem &s, const U
   else if (NB) {
     // pass 2 payload for Coulomb / Lennard-Jones alone: charge in w1
     for (int slot = team.rank(); slot < nslots; slot += team.size()) {
-      float4 pa = s.pa[slot];
       const float4 prm = s.prm[slot];
-      pa.w = prm.x;
-      s.gbv[slot].y = prm.y;     // the Lennard-Jones code, where pass 2 reads it
-      s.pa[slot] = pa;
+      slotValue(s.pb, slot, 2) = prm.x;
+      slotValue(s.pg, slot, 2) = prm.y;     // the Lennard-Jones code, where pass 2 reads it
     }
     team.sync();
   }
@@ -1773,11 +1992,6 @@ __device__ void evaluateStaged(const DevSynthesis &d, const UnitSmem &s, const U
     for (int slot = team.rank(); slot < nslots; slot += team.size()) {
       const int k = findOwner(s.slot0, nsys_u, slot);
       const int a = slot - s.slot0[k];
-      const float4 prm = s.prm[slot];
-      float4 pa = s.pa[slot];
-      float4 pb = s.pb[slot];
-      pa.w = prm.w;   // s * rho
-      pb.w = prm.z;   // rho
       float sde = 0.0f;
       if (a < s.natom[k]) {
         const int gi = d.atom_start[s.sys[k]] + a;
@@ -1792,9 +2006,8 @@ __device__ void evaluateStaged(const DevSynthesis &d, const UnitSmem &s, const U
           d.sumdeijda_ovrf[gi] = 0;
         }
       }
-      s.pa[slot] = pa;
-      s.pb[slot] = pb;
-      s.gbv[slot].y = sde;
+      // pass 3 takes the separations and dE/dR alone
+      slotValue(s.pg, slot, 2) = sde;
     }
     team.sync();
     gbDerivativeTiles(d, s, nsys_u, ntiles, us.tile_base, team.warp(), team.warps());

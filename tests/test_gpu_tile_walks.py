@@ -1,0 +1,62 @@
+"""The packed tile walks at the sizes where their lanes run out: last blocks of 1, 15, 16, 17, 31
+and 32 atoms, alone and behind full blocks, on the fused and the tiled path, and the list of
+overlapping pairs beyond its 128 entries.  Energies and forces are held to the tolerances of
+fixtures.py.
+
+Contracted molecules (coordinates scaled until most pairs of a tile overlap) are compared by psi,
+the descreening sums: every pair adds with the same sign, a pair's FP32 evaluation errs by some
+3e-7 of its closed form's terms (about a dozen roundings of 6e-8), the terms are at most about
+twelve times the integral they cancel to, and the workspace is read on a 2^-24 grid (plus a 2^-30
+rounding per partner), hence 4e-6 |psi| + 1e-7."""
+import copy
+
+import numpy as np
+import pytest
+
+import oracle
+import stormm_b200 as sb
+from fixtures import FORCE_TOL, check_energies, oracle_magnitudes, rms_rel
+from stormm_b200 import synthetic
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [2, 15, 16, 17, 31, 32, 33, 47, 48, 49, 63, 64, 65, 80, 81, 112, 129]
+
+
+@pytest.mark.parametrize("route", ["fused", "tiled"])
+def test_block_edges_match_the_oracle(route):
+    mols = [synthetic.make_molecule(4000 + n, n) for n in SIZES]
+    opts = dict(tiled_above_atoms=32) if route == "tiled" else {}
+    syn = sb.Synthesis(mols, **opts)
+    syn.set_coordinates(np.concatenate([m.coords for m in mols]))
+    syn.initialize()
+    syn.evaluate()
+    e, f = syn.energy_terms(), syn.split(syn.forces())
+    syn.initialize()
+    syn.evaluate(force=False)
+    alone = syn.energy_terms()
+    for k, m in enumerate(mols):
+        ref = oracle.from_molecule(m).evaluate(m.coords)
+        rss = oracle_magnitudes(m)
+        check_energies(e[k], ref["energies"], rss, (route, m.natom))
+        check_energies(alone[k], ref["energies"], rss, (route, m.natom, "energy only"))
+        assert rms_rel(f[k], ref["forces"]) <= FORCE_TOL, (route, m.natom)
+    syn.close()
+
+
+@pytest.mark.parametrize("route", ["fused", "tiled"])
+@pytest.mark.parametrize("natom,scale", [(16, 0.2), (40, 0.25), (64, 0.15), (97, 0.3)])
+def test_overlapping_pairs_beyond_the_list(route, natom, scale):
+    m = copy.deepcopy(synthetic.make_molecule(4100 + natom, natom))
+    m.coords = m.coords * scale
+    opts = dict(tiled_above_atoms=32) if route == "tiled" else {}
+    ref = oracle.from_molecule(m).evaluate(m.coords)
+    syn = sb.Synthesis([m], **opts)
+    syn.set_coordinates(m.coords)
+    for force in (True, False):
+        syn.initialize()
+        syn.evaluate(terms=sb.TERM_GB, force=force)
+        psi = syn.gb_workspace()[0]
+        err = np.abs(psi - ref["psi"])
+        assert np.all(err <= 4.0e-6 * np.abs(ref["psi"]) + 1.0e-7), (force, err.max())
+    syn.close()
