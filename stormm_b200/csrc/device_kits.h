@@ -23,12 +23,24 @@ constexpr int kTile = 32;                 // atoms per tile edge (one warp lane 
 constexpr int kMaxUnitSystems = 32;       // systems per fused work unit
 constexpr int kMaxFusedAtoms = 2048;      // largest molecule the fused path holds on chip
 constexpr int kNrgStride = 16;            // energy slots per system (STORMM StateVariable order)
-constexpr int kUnitMetaFields = 8;        // ints per unit-molecule row of DevSynthesis::unit_meta
+constexpr int kUnitMetaFields = 16;       // ints per unit-molecule row of DevSynthesis::unit_meta
 constexpr int kPairDerivPerTile = 512;   // float4 entries per tile of DevSynthesis::pair_deriv
 constexpr float kGbRadiiOffset = 0.09f;   // Constants/generalized_born.h:114
 constexpr float kGbKscale = 0.73f;        // Constants/generalized_born.h:123
 constexpr int kPsiBits = 29;              // fixed-point bits of the in-block psi accumulators
 constexpr int kDeijdaBits = 23;           // fixed-point bits of the in-block dE/dR accumulators
+
+// Fields of a unit molecule's row: everything a block needs to know of its molecules, so that no
+// step of an evaluation waits on a chain of loads through the per-system arrays
+enum UnitMetaField : int {
+  kMetaSystem = 0, kMetaAtoms, kMetaSlot, kMetaTile, kMetaLj,    // system, atoms; first slot, tile
+                                                                 // and table entry in the unit
+  kMetaBondChunk, kMetaAnglChunk, kMetaDiheChunk,                // first chunks of 32 terms
+  kMetaAtom0, kMetaMask0, kMetaLjTable, kMetaTypes,              // atom_start, tile_start, lj_start;
+                                                                 // types | terms in the last bond,
+                                                                 // angle, dihedral chunk << 8, 14, 20
+  kMetaBond0, kMetaAngl0, kMetaDihe0                             // bond_start, angl_start, dihe_start
+};
 
 // Energy slots (Potential/energy_enumerators.h:36-50)
 enum NrgSlot : int {
@@ -87,7 +99,6 @@ struct DevSynthesis {
 
   // tables
   const float2* ljab;            // (A, B) per type pair
-  const float2* ljab14;
   const uint4* bonds;
   const uint4* angles;
   const uint4* dihe_a;
@@ -114,10 +125,10 @@ struct DevSynthesis {
   int nunit;
   const int4* unit_desc;         // x = first row in unit_meta, y = system count,
                                  // z = atom slots (sum of padded sizes), w = tile count
-  const int* unit_meta;          // kUnitMetaFields ints per unit molecule plus a closing row per
-                                 // unit (unit_desc.x is the first row): system, atoms, first
-                                 // slot, first tile, LJ table offset, bond / angle / dihedral
-                                 // chunk offsets; the closing row holds the totals
+  const int* unit_meta;          // one row of UnitMetaField per unit molecule plus a closing row
+                                 // per unit (unit_desc.x is the first row); the closing row holds
+                                 // the totals of the prefix sums and, in kMetaSystem, the unit's
+                                 // first tile in the pair-derivative store
   int max_unit_slots;
   // HCT pair derivatives of the work units' tiles, written by GB pass 1 of a force evaluation
   // and read by pass 3: 16 steps x 32 lanes of the two pairs' i-side values, then their j-side

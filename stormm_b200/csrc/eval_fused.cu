@@ -56,7 +56,7 @@ __device__ __forceinline__ void evalFusedUnits(const DevSynthesis &d, int unit_b
         s.neck[slot] = slotNeck(d, s, k, a);
       }
       const bool real = a < s.natom[k];
-      const int gi = d.atom_start[s.sys[k]] + (real ? a : 0);
+      const int gi = unitMeta(s, kMetaAtom0, k) + (real ? a : 0);
       placeSlot(d, s, slot, real, real ? d.xcrd[gi] : 0ll, real ? d.ycrd[gi] : 0ll,
                 real ? d.zcrd[gi] : 0ll);
     }
@@ -69,7 +69,7 @@ __device__ __forceinline__ void evalFusedUnits(const DevSynthesis &d, int unit_b
         const int k = findOwner(s.slot0, us.nsys, slot);
         const int a = slot - s.slot0[k];
         if (a >= s.natom[k]) continue;
-        const int gi = d.atom_start[s.sys[k]] + a;
+        const int gi = unitMeta(s, kMetaAtom0, k) + a;
         addInt95(int63ToLong(s.fx[slot], s.fxo[slot]), &d.xfrc[gi], &d.xfrc_ovrf[gi]);
         addInt95(int63ToLong(s.fy[slot], s.fyo[slot]), &d.yfrc[gi], &d.yfrc_ovrf[gi]);
         addInt95(int63ToLong(s.fz[slot], s.fzo[slot]), &d.zfrc[gi], &d.zfrc_ovrf[gi]);

@@ -108,7 +108,7 @@ __device__ void placeUnit(const DevSynthesis &d, const DevMinimizer &m, const Un
     const int k = findOwner(s.slot0, us.nsys, slot);
     const int a = slot - s.slot0[k];
     const bool real = a < s.natom[k];
-    const int gi = d.atom_start[s.sys[k]] + (real ? a : 0);
+    const int gi = unitMeta(s, kMetaAtom0, k) + (real ? a : 0);
     placeSlot(d, s, slot, real, real ? m.xcrd[gi] : 0ll, real ? m.ycrd[gi] : 0ll,
               real ? m.zcrd[gi] : 0ll);
   }
@@ -124,7 +124,7 @@ __device__ void moveUnit(const DevSynthesis &d, const DevMinimizer &m, const Uni
     const int a = slot - s.slot0[k];
     const double step = molValue(ms, kStep, k);
     if (a < s.natom[k] && step != 0.0) {
-      const int gi = d.atom_start[s.sys[k]] + a;
+      const int gi = unitMeta(s, kMetaAtom0, k) + a;
       m.xcrd[gi] += __double2ll_rn(static_cast<double>(m.xcg[gi]) * step);
       m.ycrd[gi] += __double2ll_rn(static_cast<double>(m.ycg[gi]) * step);
       m.zcrd[gi] += __double2ll_rn(static_cast<double>(m.zcg[gi]) * step);
@@ -156,7 +156,7 @@ __device__ void minimizationCycle(const DevSynthesis &d, const DevMinimizer &m,
     const int a = slot - s.slot0[k];
     double gg = 0.0, dgg = 0.0, ff = 0.0;
     if (a < s.natom[k]) {
-      const int gi = d.atom_start[s.sys[k]] + a;
+      const int gi = unitMeta(s, kMetaAtom0, k) + a;
       const double fx = static_cast<double>(int63ToLong(s.fx[slot], s.fxo[slot]));
       const double fy = static_cast<double>(int63ToLong(s.fy[slot], s.fyo[slot]));
       const double fz = static_cast<double>(int63ToLong(s.fz[slot], s.fzo[slot]));
@@ -209,7 +209,7 @@ __device__ void minimizationCycle(const DevSynthesis &d, const DevMinimizer &m,
     const int a = slot - s.slot0[k];
     double msum = 0.0;
     if (a < s.natom[k] && ms.act[k]) {
-      const int gi = d.atom_start[s.sys[k]] + a;
+      const int gi = unitMeta(s, kMetaAtom0, k) + a;
       const long long ix = int63ToLong(s.fx[slot], s.fxo[slot]);
       const long long iy = int63ToLong(s.fy[slot], s.fyo[slot]);
       const long long iz = int63ToLong(s.fz[slot], s.fzo[slot]);

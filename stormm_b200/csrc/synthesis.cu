@@ -655,7 +655,6 @@ void Synthesis::buildLayout(const sb_topology* tops, int ntop) {
       h_ljab.push_back(make_float2(static_cast<float>(tp.lja[e]), static_cast<float>(tp.ljb[e])));
       const double a14 = (tp.lja14 != nullptr) ? tp.lja14[e] : tp.lja[e];
       const double b14 = (tp.ljb14 != nullptr) ? tp.ljb14[e] : tp.ljb[e];
-      h_ljab14.push_back(make_float2(static_cast<float>(a14), static_cast<float>(b14)));
       if (fp64) {
         h64_ljab14.push_back(make_double2(a14, b14));
         h64_ljab.push_back(make_double2(tp.lja[e], tp.ljb[e]));
@@ -864,7 +863,7 @@ std::unique_ptr<UnitPlan> Synthesis::makePlan(int max_slots_cap, int max_tiles_c
     const int nb = (atom_count[s] + kTile - 1) / kTile;
     return nb * (nb + 1) / 2;
   };
-  auto lj_of = [&](int s) { return 2 * h_lj_ntypes[s] * h_lj_ntypes[s]; };
+  auto lj_of = [&](int s) { return h_lj_ntypes[s] * h_lj_ntypes[s]; };
   const int max_lj_cap = 2048;
   std::vector<int4> &units = plan->units;
   std::vector<int> &systems = plan->systems;
@@ -936,18 +935,44 @@ void Synthesis::finalizePlan(UnitPlan* plan, bool defer) const {
       fused = fused && (tiled_index[sid] < 0);
       const int n = atom_count[sid];
       const int nblk = (n + kTile - 1) / kTile;
-      const int row[kUnitMetaFields] = {sid, n, slot, tile, lj, nb, na, nd};
+      const int bonds = h_bond_start[sid + 1] - h_bond_start[sid];
+      const int angls = h_angl_start[sid + 1] - h_angl_start[sid];
+      const int dihes = h_dihe_start[sid + 1] - h_dihe_start[sid];
+      auto last = [](int terms) { return terms > 0 ? (terms - 1) % 32 + 1 : 0; };
+      int row[kUnitMetaFields] = {};
+      row[kMetaSystem] = sid;
+      row[kMetaAtoms] = n;
+      row[kMetaSlot] = slot;
+      row[kMetaTile] = tile;
+      row[kMetaLj] = lj;
+      row[kMetaBondChunk] = nb;
+      row[kMetaAnglChunk] = na;
+      row[kMetaDiheChunk] = nd;
+      row[kMetaAtom0] = atom_start[sid];
+      row[kMetaMask0] = h_tile_start[sid];
+      row[kMetaLjTable] = h_lj_start[sid];
+      row[kMetaTypes] = h_lj_ntypes[sid] | last(bonds) << 8 | last(angls) << 14 | last(dihes) << 20;
+      row[kMetaBond0] = h_bond_start[sid];
+      row[kMetaAngl0] = h_angl_start[sid];
+      row[kMetaDihe0] = h_dihe_start[sid];
       plan->meta.insert(plan->meta.end(), row, row + kUnitMetaFields);
       slot += nblk * kTile;
       tile += nblk * (nblk + 1) / 2;
-      lj += 2 * h_lj_ntypes[sid] * h_lj_ntypes[sid];
-      nb += (h_bond_start[sid + 1] - h_bond_start[sid] + 31) / 32;
-      na += (h_angl_start[sid + 1] - h_angl_start[sid] + 31) / 32;
-      nd += (h_dihe_start[sid + 1] - h_dihe_start[sid] + 31) / 32;
+      lj += h_lj_ntypes[sid] * h_lj_ntypes[sid];
+      nb += (bonds + 31) / 32;
+      na += (angls + 31) / 32;
+      nd += (dihes + 31) / 32;
     }
     // closing row: the unit's first tile in the pair-derivative store, then the totals (units
     // of molecules on the tiled path never run the fused kernels and take no store)
-    const int last[kUnitMetaFields] = {fused ? tile_base : 0, 0, slot, tile, lj, nb, na, nd};
+    int last[kUnitMetaFields] = {};
+    last[kMetaSystem] = fused ? tile_base : 0;
+    last[kMetaSlot] = slot;
+    last[kMetaTile] = tile;
+    last[kMetaLj] = lj;
+    last[kMetaBondChunk] = nb;
+    last[kMetaAnglChunk] = na;
+    last[kMetaDiheChunk] = nd;
     plan->meta.insert(plan->meta.end(), last, last + kUnitMetaFields);
     if (slot != un.z || tile != un.w) {
       throw Error(SB_ERR_ARGUMENT, "inconsistent work-unit descriptor");
@@ -1031,7 +1056,7 @@ void Synthesis::buildUnits() {
     single_plan->systems[s] = s;
     if (tiled_index[s] < 0) {
       single_slots = std::max(single_slots, slots_of(s));
-      single_lj = std::max(single_lj, 2 * h_lj_ntypes[s] * h_lj_ntypes[s]);
+      single_lj = std::max(single_lj, h_lj_ntypes[s] * h_lj_ntypes[s]);
     }
   }
   max_unit_slots = single_slots;
@@ -1068,7 +1093,6 @@ void Synthesis::upload() {
   arena.put(&d_gb_radius64, h_gb_radius64);
   arena.put(&d_gb_gamma64, h_gb_gamma64);
   arena.put(&d_ljab, h_ljab);
-  arena.put(&d_ljab14, h_ljab14);
   arena.put(&d_bonds, h_bonds);
   arena.put(&d_angles, h_angles);
   arena.put(&d_dihe_a, h_dihe_a);
@@ -1254,7 +1278,6 @@ void Synthesis::upload() {
   d.gb_radius64 = d_gb_radius64.p;
   d.gb_gamma64 = d_gb_gamma64.p;
   d.ljab = d_ljab.p;
-  d.ljab14 = d_ljab14.p;
   d.bonds = d_bonds.p;
   d.angles = d_angles.p;
   d.dihe_a = d_dihe_a.p;

@@ -256,7 +256,7 @@ public:
   std::vector<double> h_gb_gamma64;
   std::vector<int> h_ljidx, h_lj_start, h_lj_ntypes, h_tile_start, h_tile_mask_idx;
   std::vector<int> h_bond_start, h_angl_start, h_dihe_start;
-  std::vector<float2> h_ljab, h_ljab14;
+  std::vector<float2> h_ljab;
   std::vector<uint4> h_bonds, h_angles, h_dihe_a, h_dihe_b;
   std::vector<double4> h_angl64, h_dihe64;
   std::vector<double4> h_dihe14_64;
@@ -296,7 +296,7 @@ public:
   DeviceArray<float> d_charge, d_rho, d_srho, d_pb, d_alpha, d_beta, d_gamma;
   DeviceArray<double4> d_gb_radius64;
   DeviceArray<double> d_gb_gamma64;
-  DeviceArray<float2> d_ljab, d_ljab14;
+  DeviceArray<float2> d_ljab;
   DeviceArray<uint4> d_bonds, d_angles, d_dihe_a, d_dihe_b;
   DeviceArray<double4> d_angl64, d_dihe64;
   DeviceArray<double4> d_dihe14_64;

@@ -26,19 +26,26 @@ constexpr int kStageSlots = 2 * kTile;    // block I in slots 0-31, block J in s
 // energies with global integer atomics (one molecule per block row of the launch grid)
 struct GlobalValence {
   const DevSynthesis &d;
-  const int* bchunk0;
-  const int* achunk0;
-  const int* dchunk0;
-  const int* sys;
-  const int* slot0;
-  __device__ GlobalValence(const DevSynthesis &d_in, const int* chunks, const int* sys_in,
-                           const int* slot0_in) :
-      d(d_in), bchunk0(chunks), achunk0(chunks + 2), dchunk0(chunks + 4), sys(sys_in),
-      slot0(slot0_in) {}
-  __device__ __forceinline__ int chunkBegin() const {
-    return (threadIdx.x >> 5) + blockIdx.y * (blockDim.x >> 5);
+  int sys;
+  int first;     // the molecule's first atom
+  __device__ GlobalValence(const DevSynthesis &d_in, int sys_in) :
+      d(d_in), sys(sys_in), first(d_in.atom_start[sys_in]) {}
+  __device__ __forceinline__ const int* starts(int kind) const {
+    return (kind == kBondTerms) ? d.bond_start :
+           (kind == kAnglTerms) ? d.angl_start : d.dihe_start;
+  }
+  __device__ __forceinline__ int chunks(int kind) const {
+    return (starts(kind)[sys + 1] - starts(kind)[sys] + 31) / 32;
+  }
+  __device__ __forceinline__ int begin(int before) const {
+    return dealFrom((threadIdx.x >> 5) + blockIdx.y * (blockDim.x >> 5), chunkStride(), before);
   }
   __device__ __forceinline__ int chunkStride() const { return (blockDim.x >> 5) * gridDim.y; }
+  __device__ __forceinline__ ValenceTerm term(int kind, int c, int lane) const {
+    const int index = starts(kind)[sys] + 32 * c + lane;
+    return ValenceTerm{0, index, index < starts(kind)[sys + 1]};
+  }
+  __device__ __forceinline__ int slot0(int) const { return first; }
   __device__ __forceinline__ float3 part(int i, bool high) const {
     float3 h, l;
     splitCoordinate(static_cast<double>(d.xcrd[i]) * d.inv_gpos_scale, &h.x, &l.x);
@@ -56,10 +63,10 @@ struct GlobalValence {
     atomicAdd(reinterpret_cast<unsigned long long*>(&d.zfrc[i]),
               static_cast<unsigned long long>(__float2ll_rn(fz * scale)));
   }
-  __device__ __forceinline__ void energy(int k, int slot, float e, float scale) const {
+  __device__ __forceinline__ void energy(int, int slot, float e, float scale) const {
     const long long v = warpSum(__float2ll_rn(e * scale));
     if ((threadIdx.x & 31) == 0 && v != 0) {
-      atomicAdd(&d.energies[sys[k] * kNrgStride + slot], static_cast<unsigned long long>(v));
+      atomicAdd(&d.energies[sys * kNrgStride + slot], static_cast<unsigned long long>(v));
     }
   }
   __device__ __forceinline__ double3 pos64(int i) const {
@@ -77,14 +84,14 @@ struct GlobalValence {
     atomicAdd(reinterpret_cast<unsigned long long*>(&d.zfrc[i]),
               static_cast<unsigned long long>(__double2ll_rn(fz * s)));
   }
-  __device__ __forceinline__ void energy64(int k, int slot, double e, float scale) const {
+  __device__ __forceinline__ void energy64(int, int slot, double e, float scale) const {
     const long long v = warpSum(__double2ll_rn(e * static_cast<double>(scale)));
     if ((threadIdx.x & 31) == 0 && v != 0) {
-      atomicAdd(&d.energies[sys[k] * kNrgStride + slot], static_cast<unsigned long long>(v));
+      atomicAdd(&d.energies[sys * kNrgStride + slot], static_cast<unsigned long long>(v));
     }
   }
-  __device__ __forceinline__ float2 clash(int k) const {
-    const int cycle = (d.clash_cycle != nullptr) ? d.clash_cycle[sys[k]] : -1;
+  __device__ __forceinline__ float2 clash(int) const {
+    const int cycle = (d.clash_cycle != nullptr) ? d.clash_cycle[sys] : -1;
     return clashScaled(d.clash_distance, d.clash_ratio, d.clash_cycles, cycle);
   }
 };
@@ -93,24 +100,8 @@ struct GlobalValence {
 template <bool FORCE, bool ENERGY, bool CLASH>
 __global__ void __launch_bounds__(256)
 kTiledValence(const DevSynthesis d, const DevTiled t, int mol_begin) {
-  __shared__ int sys[1];
-  __shared__ int slot0[1];
-  __shared__ int chunks[6];   // bond, angle, dihedral chunk prefix sums (0, count) each
-  const int m = mol_begin + blockIdx.x;
-  if (threadIdx.x == 0) {
-    const int s = t.systems[m];
-    sys[0] = s;
-    slot0[0] = d.atom_start[s];
-    chunks[0] = 0;
-    chunks[1] = (d.bond_start[s + 1] - d.bond_start[s] + 31) / 32;
-    chunks[2] = 0;
-    chunks[3] = (d.angl_start[s + 1] - d.angl_start[s] + 31) / 32;
-    chunks[4] = 0;
-    chunks[5] = (d.dihe_start[s + 1] - d.dihe_start[s] + 31) / 32;
-  }
-  __syncthreads();
-  const GlobalValence v(d, chunks, sys, slot0);
-  valenceTerms<FORCE, ENERGY, GlobalValence, CLASH>(d, v, 1);
+  valenceTerms<FORCE, ENERGY, GlobalValence, CLASH>(
+      d, GlobalValence(d, t.systems[mol_begin + blockIdx.x]));
 }
 
 // Stage one tile's atom blocks into a warp's slice: block I in slots 0-31, block J in 32-63

@@ -234,9 +234,10 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __
 // minimax fits on 1/16 <= t <= 0.3: relative error of the sums below 1.1e-8 and 4.3e-9).  No
 // reciprocal, logarithm or cancellation, so it is more accurate than the closed form in FP32.
 // It tells where it does not apply (overlapping spheres, or t > 0.3): bonded neighbours mostly, a
-// few pairs per atom, which hctClosed2 evaluates after the tile's walk.  Against one
-// branch per step on r <= 4 sj (nearly every step of a small molecule has such a pair on some
-// lane): HCT_NOTE
+// few pairs per atom, which hctClosed2 evaluates after the tile's walk (spreadLate), in place of
+// a branch per step on r <= 4 sj, which nearly every step of a small molecule takes on some lane
+// (with each lane evaluating its own such pairs in turn, the busiest lane, with some eight, set the
+// cost and the gain was 1 %).
 // BRANCH: the polynomial behind a branch, for tiles where most steps have no pair within 4 sj.
 constexpr float kSeriesLimit = 0.3f;
 
@@ -417,19 +418,21 @@ struct UnitSmem {
   int* de;          // int63 dE/dR accumulator, 2^kDeijdaBits
   int* deo;
   int* neck;        // neck GB table index of the atom
-  float2* lj;       // Lennard-Jones tables of the unit's molecules (standard, then 1-4)
+  float2* lj;       // Lennard-Jones tables of the unit's molecules
   unsigned long long* nrg;   // per unit molecule energies
-  int* sys;         // molecule index
-  int* slot0;       // first slot of the molecule
+  int* meta;        // the unit's rows of DevSynthesis::unit_meta by field: metaStride entries each,
+  int metaStride;   // one per molecule and the closing one
+  int* sys;         // molecule index, number of atoms, first slot: views into meta
   int* natom;
-  int* ljbase;      // prefix sums of the molecules' table sizes (kMaxUnitSystems + 1)
-  int* tile0;       // prefix sums (kMaxUnitSystems + 1 entries each)
-  int* bchunk0;     // valence work in chunks of 32 terms that never straddle two molecules
-  int* achunk0;
-  int* dchunk0;
+  int* slot0;
   float2* clash;    // per unit molecule: clash distance and sigma ratio of this evaluation
   unsigned short* late;   // kLateEntries per warp: pairs of GB pass 1 set aside (RadiiPass)
 };
+
+// Field f of unit molecule k's row (k = number of molecules: the closing row)
+__device__ __forceinline__ int unitMeta(const UnitSmem &s, int f, int k) {
+  return s.meta[f * s.metaStride + k];
+}
 
 // Atom pair records: slot s of a unit is atom (s / 16) % 2 of record 16 (s / 32) + s % 16
 constexpr int kRecords = kTile / 2;
@@ -488,7 +491,7 @@ __host__ __device__ inline size_t unitSmemBytes(int max_slots, int max_lj,
   b = alignUp(b, 16);
   b += sizeof(unsigned long long) * max_sys * kNrgStride;
   b += sizeof(float2) * max_sys;
-  b += sizeof(int) * (3 * max_sys + 5 * (max_sys + 1));
+  b += sizeof(int) * kUnitMetaFields * (max_sys + 1);
   b += sizeof(unsigned short) * kLateEntries * kLateWarps;
   return alignUp(b, 16);
 }
@@ -524,14 +527,12 @@ __device__ UnitSmem carveSmem(char* base, int max_slots, int max_lj,
   s.clash = reinterpret_cast<float2*>(base + off);
   off += sizeof(float2) * max_sys;
   int* q = reinterpret_cast<int*>(base + off);
-  s.sys = q; q += max_sys;
-  s.slot0 = q; q += max_sys;
-  s.natom = q; q += max_sys;
-  s.ljbase = q; q += max_sys + 1;
-  s.tile0 = q; q += max_sys + 1;
-  s.bchunk0 = q; q += max_sys + 1;
-  s.achunk0 = q; q += max_sys + 1;
-  s.dchunk0 = q; q += max_sys + 1;
+  s.meta = q;
+  s.metaStride = max_sys + 1;
+  s.sys = q + kMetaSystem * (max_sys + 1);
+  s.natom = q + kMetaAtoms * (max_sys + 1);
+  s.slot0 = q + kMetaSlot * (max_sys + 1);
+  q += kUnitMetaFields * (max_sys + 1);
   s.late = reinterpret_cast<unsigned short*>(q);
   return s;
 }
@@ -620,21 +621,51 @@ __device__ __forceinline__ void warpEnergy(const UnitSmem &s, int k, int slot, f
 // Valence terms (Potential/valence_potential.tpp).  Warps take chunks of 32 terms of one molecule,
 // so each chunk's energies reduce across the warp into a single shared-memory update.
 // ------------------------------------------------------------------------------------------------
-// Where valence terms read their atoms and put forces and energies: a work unit's shared memory
+// The three kinds of valence terms, taken in chunks of 32 that never straddle two molecules
+enum ValenceKind : int { kBondTerms = 0, kAnglTerms, kDiheTerms };
+
+// A lane's term of a chunk: its molecule, its index in the synthesis' list, and whether the chunk
+// reaches this lane
+struct ValenceTerm {
+  int k;
+  int index;
+  bool valid;
+};
+
+// First item of a list for rank r of n that take it in turn, when `before` items of other lists
+// have been dealt out before it: the ranks that took one item less come first
+__device__ __forceinline__ int dealFrom(int r, int n, int before) {
+  const int v = (r - before) % n;
+  return v < 0 ? v + n : v;
+}
+
+// Where valence terms read their atoms and put forces and energies: a work unit's shared memory.
+// The chunks of the three kinds are dealt to the warps in one sequence, as are the GB tiles after
+// them, so that a small molecule's dihedrals, angles, bonds and tiles run on different warps side
+// by side and not on the first warps one after another (with the molecule table of a unit read in
+// one step: 60 minimization cycles of one 48-atom molecule 6.20 -> 5.18 ms, 384 molecules of 20-200
+// atoms 165 -> 159 us).
 struct SmemValence {
   const UnitSmem &s;
-  const int* bchunk0;
-  const int* achunk0;
-  const int* dchunk0;
-  const int* sys;
-  const int* slot0;
-  int begin;
+  int nsys;
+  int rank;
   int stride;
-  __device__ SmemValence(const UnitSmem &s_in, int begin_in, int stride_in) :
-      s(s_in), bchunk0(s_in.bchunk0), achunk0(s_in.achunk0), dchunk0(s_in.dchunk0),
-      sys(s_in.sys), slot0(s_in.slot0), begin(begin_in), stride(stride_in) {}
-  __device__ __forceinline__ int chunkBegin() const { return begin; }
+  __device__ SmemValence(const UnitSmem &s_in, int nsys_in, int rank_in, int stride_in) :
+      s(s_in), nsys(nsys_in), rank(rank_in), stride(stride_in) {}
+  __device__ __forceinline__ int chunks(int kind) const {
+    return unitMeta(s, kMetaBondChunk + kind, nsys);
+  }
+  __device__ __forceinline__ int begin(int before) const { return dealFrom(rank, stride, before); }
   __device__ __forceinline__ int chunkStride() const { return stride; }
+  __device__ __forceinline__ ValenceTerm term(int kind, int c, int lane) const {
+    const int* first = s.meta + (kMetaBondChunk + kind) * s.metaStride;
+    const int k = findOwner(first, nsys, c);
+    const int rel = c - first[k];
+    const int tail = (unitMeta(s, kMetaTypes, k) >> (8 + 6 * kind)) & 63;
+    const int here = (c + 1 == first[k + 1]) ? tail : 32;
+    return ValenceTerm{k, unitMeta(s, kMetaBond0 + kind, k) + 32 * rel + lane, lane < here};
+  }
+  __device__ __forceinline__ int slot0(int k) const { return s.slot0[k]; }
   __device__ __forceinline__ float3 hi(int i) const { return slotHi(s, i); }
   __device__ __forceinline__ float3 lo(int i) const { return slotLo(s, i); }
   __device__ __forceinline__ void force(int i, float fx, float fy, float fz, float scale) const {
@@ -666,23 +697,23 @@ struct SmemValence {
 };
 
 template <bool FORCE, bool ENERGY, class V, bool CLASH = false>
-__device__ void valenceTerms(const DevSynthesis &d, const V &v, int nsys_u) {
+__device__ void valenceTerms(const DevSynthesis &d, const V &v) {
   const float fs = d.frc_scale;
   const float es = d.nrg_scale;
   const int lane = threadIdx.x & 31;
+  const int nbond = v.chunks(kBondTerms), nangl = v.chunks(kAnglTerms);
+  const int ndihe = v.chunks(kDiheTerms);
 
   // bonds, valence_potential.tpp:9-97; the equilibrium length is a float pair so that r - r0
   // loses nothing to the rounding of r0, and the bond length itself is an unevaluated pair
-  for (int c = v.chunkBegin(); c < v.bchunk0[nsys_u]; c += v.chunkStride()) {
-    const int k = findOwner(v.bchunk0, nsys_u, c);
-    const int sysid = v.sys[k];
-    const int t = (c - v.bchunk0[k]) * 32 + lane;
-    const int nterm = d.bond_start[sysid + 1] - d.bond_start[sysid];
+  for (int c = v.begin(ndihe + nangl); c < nbond; c += v.chunkStride()) {
+    const ValenceTerm t = v.term(kBondTerms, c, lane);
+    const int k = t.k;
     float e = 0.0f;
-    if (t < nterm) {
-      const uint4 rec = d.bonds[d.bond_start[sysid] + t];
-      const int ia = v.slot0[k] + static_cast<int>(rec.x & 0xffffu);
-      const int ja = v.slot0[k] + static_cast<int>(rec.x >> 16);
+    if (t.valid) {
+      const uint4 rec = d.bonds[t.index];
+      const int ia = v.slot0(k) + static_cast<int>(rec.x & 0xffffu);
+      const int ja = v.slot0(k) + static_cast<int>(rec.x >> 16);
       const float keq = __uint_as_float(rec.y);
       const float leq_hi = __uint_as_float(rec.z);
       const float leq_lo = __uint_as_float(rec.w);
@@ -731,18 +762,16 @@ __device__ void valenceTerms(const DevSynthesis &d, const V &v, int nsys_u) {
   // angle's force divides by sin(theta), which FP32 deltas and cross products only give to
   // about 1e-7 absolute.  theta - theta0 comes from rotating (cos, sin) of theta, taken from the
   // dot and cross products, by theta0: well conditioned everywhere.
-  for (int c = v.chunkBegin(); c < v.achunk0[nsys_u]; c += v.chunkStride()) {
-    const int k = findOwner(v.achunk0, nsys_u, c);
-    const int sysid = v.sys[k];
-    const int t = (c - v.achunk0[k]) * 32 + lane;
-    const int nterm = d.angl_start[sysid + 1] - d.angl_start[sysid];
+  for (int c = v.begin(ndihe); c < nangl; c += v.chunkStride()) {
+    const ValenceTerm t = v.term(kAnglTerms, c, lane);
+    const int k = t.k;
     double e = 0.0;
-    if (t < nterm) {
-      const uint4 rec = d.angles[d.angl_start[sysid] + t];
-      const double4 prm = d.angl64[d.angl_start[sysid] + t];   // k, cos, sin, theta0
-      const int ia = v.slot0[k] + static_cast<int>(rec.x & 0xffffu);
-      const int ja = v.slot0[k] + static_cast<int>(rec.x >> 16);
-      const int ka = v.slot0[k] + static_cast<int>(rec.y);
+    if (t.valid) {
+      const uint4 rec = d.angles[t.index];
+      const double4 prm = d.angl64[t.index];   // k, cos, sin, theta0
+      const int ia = v.slot0(k) + static_cast<int>(rec.x & 0xffffu);
+      const int ja = v.slot0(k) + static_cast<int>(rec.x >> 16);
+      const int ka = v.slot0(k) + static_cast<int>(rec.y);
       const double3 pj = v.pos64(ja);
       const double3 ba = sub3d(v.pos64(ia), pj);
       const double3 bc = sub3d(v.pos64(ka), pj);
@@ -788,23 +817,20 @@ __device__ void valenceTerms(const DevSynthesis &d, const V &v, int nsys_u) {
   // and sin(n theta - phase) follow from the multiple-angle recurrence for integer
   // periodicities.  1 + cos(psi) cancels near psi = pi (impropers, and propers near their
   // minimum); there sin^2(psi) / (1 - cos(psi)) gives the same value without the cancellation.
-  for (int c = v.chunkBegin(); c < v.dchunk0[nsys_u]; c += v.chunkStride()) {
-    const int k = findOwner(v.dchunk0, nsys_u, c);
-    const int sysid = v.sys[k];
-    const int t = (c - v.dchunk0[k]) * 32 + lane;
-    const int nterm = d.dihe_start[sysid + 1] - d.dihe_start[sysid];
+  for (int c = v.begin(0); c < ndihe; c += v.chunkStride()) {
+    const ValenceTerm t = v.term(kDiheTerms, c, lane);
+    const int k = t.k;
     double e_prop = 0.0, e_impr = 0.0, e_el14 = 0.0, e_lj14 = 0.0;
-    if (t < nterm) {
-      const int pos = d.dihe_start[sysid] + t;
-      const uint4 ra = d.dihe_a[pos];
-      const double4 prm = d.dihe64[pos];     // amplitude, cos(phase), sin(phase), periodicity
-      const double4 p14 = d.dihe14_64[pos];  // the attached 1-4 pair: q q / scee, A, B, flag
+    if (t.valid) {
+      const uint4 ra = d.dihe_a[t.index];
+      const double4 prm = d.dihe64[t.index];     // amplitude, cos(phase), sin(phase), periodicity
+      const double4 p14 = d.dihe14_64[t.index];  // the attached 1-4 pair: q q / scee, A, B, flag
       const int li = static_cast<int>(ra.x & 0xffffu);
       const int ll = static_cast<int>((ra.y >> 16) & 0x7fffu);
-      const int ia = v.slot0[k] + li;
-      const int ja = v.slot0[k] + static_cast<int>(ra.x >> 16);
-      const int ka = v.slot0[k] + static_cast<int>(ra.y & 0xffffu);
-      const int la = v.slot0[k] + ll;
+      const int ia = v.slot0(k) + li;
+      const int ja = v.slot0(k) + static_cast<int>(ra.x >> 16);
+      const int ka = v.slot0(k) + static_cast<int>(ra.y & 0xffffu);
+      const int la = v.slot0(k) + ll;
       const bool improper = (ra.y & 0x80000000u) != 0u;
       const double3 pi = v.pos64(ia);
       const double3 pj = v.pos64(ja);
@@ -935,8 +961,8 @@ struct TileInfo {
 
 __device__ __forceinline__ TileInfo tileInfo(const UnitSmem &s, int nsys_u, int t) {
   TileInfo ti;
-  ti.k = findOwner(s.tile0, nsys_u, t);
-  ti.local = t - s.tile0[ti.k];
+  ti.k = findOwner(s.meta + kMetaTile * s.metaStride, nsys_u, t);
+  ti.local = t - unitMeta(s, kMetaTile, ti.k);
   int I, J;
   tileCoordinates(ti.local, &I, &J);
   const int n = s.natom[ti.k];
@@ -1654,7 +1680,7 @@ __device__ void pairTiles(const DevSynthesis &d, const UnitSmem &s, int nsys_u, 
     }
     unsigned mask = 0u;
     if (NB) {
-      const int midx = d.tile_mask_idx[d.tile_start[s.sys[ti.k]] + ti.local];
+      const int midx = d.tile_mask_idx[unitMeta(s, kMetaMask0, ti.k) + ti.local];
       if (midx != 0) {
         mask = __ldg(&d.mask_pool[static_cast<size_t>(midx) * 32 + w.il]);
       }
@@ -1796,38 +1822,24 @@ __device__ bool stageUnitTables(const DevSynthesis &d, const UnitSmem &s, int u,
     }
     return false;
   }
-  // the unit's molecule table, precomputed on the host: one coalesced load per field
+  // the unit's molecule table, precomputed on the host
   const int* meta = d.unit_meta + static_cast<size_t>(desc.x) * kUnitMetaFields;
-  shape->tile_base = meta[nsys_u * kUnitMetaFields];
+  shape->tile_base = meta[nsys_u * kUnitMetaFields + kMetaSystem];
   for (int e = team.rank(); e < (nsys_u + 1) * kUnitMetaFields; e += team.size()) {
-    const int k = e / kUnitMetaFields;
-    const int v = meta[e];
-    switch (e % kUnitMetaFields) {
-      case 0: if (k < nsys_u) s.sys[k] = v; break;
-      case 1: if (k < nsys_u) s.natom[k] = v; break;
-      case 2: if (k < nsys_u) s.slot0[k] = v; break;
-      case 3: s.tile0[k] = v; break;
-      case 4: s.ljbase[k] = v; break;
-      case 5: s.bchunk0[k] = v; break;
-      case 6: s.achunk0[k] = v; break;
-      default: s.dchunk0[k] = v; break;
-    }
+    s.meta[(e % kUnitMetaFields) * s.metaStride + e / kUnitMetaFields] = meta[e];
   }
   team.sync();
-  if (desc.z > d.max_unit_slots || s.ljbase[nsys_u] > max_lj || nsys_u > max_sys) {
+  const int nlj = unitMeta(s, kMetaLj, nsys_u);
+  if (desc.z > d.max_unit_slots || nlj > max_lj || nsys_u > max_sys) {
     if (team.rank() == 0) {
       atomicOr(d.status, 1);
     }
     return false;   // reported through the status word; nothing in the unit is touched
   }
-  // Lennard-Jones tables (standard then 1-4) of every molecule, all entries in parallel
-  for (int e = team.rank(); e < s.ljbase[nsys_u]; e += team.size()) {
-    const int k = findOwner(s.ljbase, nsys_u, e);
-    const int sysid = s.sys[k];
-    const int nt = d.lj_ntypes[sysid];
-    const int rel = e - s.ljbase[k];
-    const int src = d.lj_start[sysid] + (rel < nt * nt ? rel : rel - nt * nt);
-    s.lj[e] = (rel < nt * nt) ? d.ljab[src] : d.ljab14[src];
+  // Lennard-Jones tables of every molecule, all entries in parallel
+  for (int e = team.rank(); e < nlj; e += team.size()) {
+    const int k = findOwner(s.meta + kMetaLj * s.metaStride, nsys_u, e);
+    s.lj[e] = d.ljab[unitMeta(s, kMetaLjTable, k) + e - unitMeta(s, kMetaLj, k)];
   }
   team.sync();
   return true;
@@ -1839,19 +1851,19 @@ __device__ bool stageUnitTables(const DevSynthesis &d, const UnitSmem &s, int u,
 __device__ __forceinline__ float4 slotParameters(const DevSynthesis &d, const UnitSmem &s, int k,
                                                  int a) {
   if (a < s.natom[k]) {
-    const int sysid = s.sys[k];
-    const int gi = d.atom_start[sysid] + a;
-    const int nt = d.lj_ntypes[sysid];
+    const int gi = unitMeta(s, kMetaAtom0, k) + a;
+    const int nt = unitMeta(s, kMetaTypes, k) & 0xff;
     const int ty = d.lj_idx[gi];
-    return make_float4(d.charge[gi], __int_as_float((s.ljbase[k] + ty * nt) | (ty << 16)),
+    return make_float4(d.charge[gi],
+                       __int_as_float((unitMeta(s, kMetaLj, k) + ty * nt) | (ty << 16)),
                        d.rho[gi], d.srho[gi]);
   }
-  return make_float4(0.0f, __int_as_float(s.ljbase[k]), 1.0f, 0.0f);
+  return make_float4(0.0f, __int_as_float(unitMeta(s, kMetaLj, k)), 1.0f, 0.0f);
 }
 
 // Neck GB table index of slot a of unit molecule k (0 for padding or other GB models)
 __device__ __forceinline__ int slotNeck(const DevSynthesis &d, const UnitSmem &s, int k, int a) {
-  return (d.neck_size > 0 && a < s.natom[k]) ? d.neck_idx[d.atom_start[s.sys[k]] + a] : 0;
+  return (d.neck_size > 0 && a < s.natom[k]) ? d.neck_idx[unitMeta(s, kMetaAtom0, k) + a] : 0;
 }
 
 // Write a slot's coordinates, payloads and GB values
@@ -1914,14 +1926,18 @@ __device__ void evaluateStaged(const DevSynthesis &d, const UnitSmem &s, const U
 
   // valence terms and GB pass 1 touch disjoint accumulators: no barrier between them
   if (VALE) {
-    valenceTerms<FORCE, ENERGY, SmemValence, CLASH>(d, SmemValence(s, team.warp(), team.warps()),
-                                                    nsys_u);
+    valenceTerms<FORCE, ENERGY, SmemValence, CLASH>(
+        d, SmemValence(s, nsys_u, team.warp(), team.warps()));
     if (!gb) {
       team.sync();
     }
   }
   if (gb) {
-    gbRadiiTiles<FORCE, NECK>(d, s, nsys_u, ntiles, us.tile_base, team.warp(), team.warps());
+    const int dealt = VALE ? unitMeta(s, kMetaBondChunk, nsys_u) +
+                             unitMeta(s, kMetaAnglChunk, nsys_u) +
+                             unitMeta(s, kMetaDiheChunk, nsys_u) : 0;
+    gbRadiiTiles<FORCE, NECK>(d, s, nsys_u, ntiles, us.tile_base,
+                              dealFrom(team.warp(), team.warps(), dealt), team.warps());
     team.sync();
     // effective radii, self terms (nonbonded_potential.tpp:730-805); a warp's 32 slots
     // belong to one molecule, so the self energies reduce across the warp
@@ -1934,7 +1950,7 @@ __device__ void evaluateStaged(const DevSynthesis &d, const UnitSmem &s, const U
       const float4 prm = s.prm[slot];
       float egbi = 1.0f;
       if (a < s.natom[k]) {
-        const int gi = d.atom_start[s.sys[k]] + a;
+        const int gi = unitMeta(s, kMetaAtom0, k) + a;
         const double psi = static_cast<double>(int63ToLong(s.psi[slot], s.psio[slot])) *
                            static_cast<double>(inv_ps);
         egbi = effectiveRadius(d, gi, psi);
@@ -1994,7 +2010,7 @@ __device__ void evaluateStaged(const DevSynthesis &d, const UnitSmem &s, const U
       const int a = slot - s.slot0[k];
       float sde = 0.0f;
       if (a < s.natom[k]) {
-        const int gi = d.atom_start[s.sys[k]] + a;
+        const int gi = unitMeta(s, kMetaAtom0, k) + a;
         sde = static_cast<float>(int63ToLong(s.de[slot], s.deo[slot])) * inv_ds;
         if (d.igb != 1) {
           const double psi = static_cast<double>(int63ToLong(s.psi[slot], s.psio[slot])) *
