@@ -134,7 +134,7 @@ __device__ void moveUnit(const DevSynthesis &d, const DevMinimizer &m, const Uni
 
 // One line-minimization cycle of every unit molecule that has not converged; with CLASH, the
 // four evaluations of a molecule still within m.clash_cycles use softened cores
-template <bool HIST, bool CLASH, bool NECK, class Team>
+template <bool CLASH, bool NECK, class Team>
 __device__ void minimizationCycle(const DevSynthesis &d, const DevMinimizer &m,
                                   const UnitSmem &s, const MinSmem &ms, const UnitShape &us,
                                   const Team &team) {
@@ -189,7 +189,7 @@ __device__ void minimizationCycle(const DevSynthesis &d, const DevMinimizer &m,
     if (ms.act[k]) {
       const double rms = sqrt(ff / (3.0 * static_cast<double>(s.natom[k])));
       m.rms_force[sysid] = rms;
-      if (HIST && ms.cyc[k] < m.hist_stride) {
+      if (m.history != nullptr && ms.cyc[k] < m.hist_stride) {
         m.history[static_cast<size_t>(sysid) * m.hist_stride + ms.cyc[k]] = e0;
       }
       if (m.drms > 0.0 && rms <= m.drms) {
@@ -323,7 +323,7 @@ __device__ void minimizationCycle(const DevSynthesis &d, const DevMinimizer &m,
 }
 
 // Every cycle of one work unit, then its final energies (undamped) and state
-template <bool HIST, bool CLASH, bool NECK, class Team>
+template <bool CLASH, bool NECK, class Team>
 __device__ void minimizeUnit(const DevSynthesis &d, const DevMinimizer &m, const UnitSmem &s,
                              const MinSmem &ms, int u, int max_lj, int max_sys, int cycles,
                              int final_energy, const Team &team) {
@@ -356,7 +356,7 @@ __device__ void minimizeUnit(const DevSynthesis &d, const DevMinimizer &m, const
     if (!team.any(moving != 0)) {
       break;
     }
-    minimizationCycle<HIST, CLASH, NECK>(d, m, s, ms, us, team);
+    minimizationCycle<CLASH, NECK>(d, m, s, ms, us, team);
   }
   if (final_energy) {
     // one more energy evaluation at the final coordinates (hpc_minimization.cu:372-383)
@@ -365,7 +365,7 @@ __device__ void minimizeUnit(const DevSynthesis &d, const DevMinimizer &m, const
     for (int e = team.rank(); e < us.nsys * kNrgStride; e += team.size()) {
       d.energies[s.sys[e / kNrgStride] * kNrgStride + (e % kNrgStride)] = s.nrg[e];
     }
-    if (HIST && team.rank() < us.nsys) {
+    if (m.history != nullptr && team.rank() < us.nsys) {
       const int k = team.rank();
       if (ms.cyc[k] < m.hist_stride) {
         m.history[static_cast<size_t>(s.sys[k]) * m.hist_stride + ms.cyc[k]] =
@@ -385,9 +385,10 @@ __device__ void minimizeUnit(const DevSynthesis &d, const DevMinimizer &m, const
 
 // One thread block per work unit (molecules of up to 2,048 atoms).  The minimizer keeps more
 // state live than a single evaluation; two blocks per SM with up to 128 registers a thread run
-// faster than four with 64, where the pair loops spill.
-template <bool HIST, bool CLASH, bool NECK>
-__global__ void __launch_bounds__(256, 2)
+// faster than four with 64, where the pair loops spill.  THREADS 512: one block per SM, for
+// launches of at most that many units.
+template <bool CLASH, bool NECK, int THREADS>
+__global__ void __launch_bounds__(THREADS, 512 / THREADS)
 kMinimize(const DevSynthesis d, const DevMinimizer m, int unit_begin, int unit_end, int max_lj,
           int cycles, int final_energy) {
   extern __shared__ __align__(16) char smem_raw[];
@@ -398,7 +399,7 @@ kMinimize(const DevSynthesis d, const DevMinimizer m, int unit_begin, int unit_e
   const BlockTeam team;
   int u = unit_begin + blockIdx.x;
   while (u < unit_end) {
-    minimizeUnit<HIST, CLASH, NECK>(d, m, s, ms, u, max_lj, kMaxUnitSystems, cycles,
+    minimizeUnit<CLASH, NECK>(d, m, s, ms, u, max_lj, kMaxUnitSystems, cycles,
                                     final_energy, team);
     if (threadIdx.x == 0) {
       next_unit = unit_begin + static_cast<int>(gridDim.x) + atomicAdd(m.queue, 1);
@@ -458,12 +459,13 @@ cudaError_t launchMinimize(const DevSynthesis &d, const DevMinimizer &m, int uni
   const size_t smem = minimizeSmemBytes(d.max_unit_slots, max_lj);
   const bool clash = m.clash_cycles > 0 && (m.clash_distance > 0.0f || m.clash_ratio > 0.0f);
   const bool neck = d.neck_size > 0;
-  auto pick = [&](auto hist) {
-    constexpr bool H = decltype(hist)::value;
-    return neck ? (clash ? kMinimize<H, true, true> : kMinimize<H, false, true>) :
-                  (clash ? kMinimize<H, true, false> : kMinimize<H, false, false>);
+  auto pick = [&](auto threads_c) {
+    constexpr int T = decltype(threads_c)::value;
+    return neck ? (clash ? kMinimize<true, true, T> : kMinimize<false, true, T>) :
+                  (clash ? kMinimize<true, false, T> : kMinimize<false, false, T>);
   };
-  auto kern = (m.history != nullptr) ? pick(std::true_type()) : pick(std::false_type());
+  auto kern = (threads > 256) ? pick(std::integral_constant<int, 512>()) :
+                                pick(std::integral_constant<int, 256>());
   cudaError_t err = allowLargeSmem(kern);
   if (err != cudaSuccess) return err;
   int per_sm = 0;

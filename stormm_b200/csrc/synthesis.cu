@@ -880,6 +880,7 @@ std::unique_ptr<UnitPlan> Synthesis::makePlan(int max_slots_cap, int max_tiles_c
     systems.push_back(s);
     plan->big_slots = std::max(plan->big_slots, slots_of(s));
     plan->big_lj = std::max(plan->big_lj, lj_of(s));
+    plan->big_tiles += tiles_of(s);
     plan->n_big++;
     first_small++;
   }
@@ -898,6 +899,7 @@ std::unique_ptr<UnitPlan> Synthesis::makePlan(int max_slots_cap, int max_tiles_c
       cur_lj = 0;
     }
     systems.push_back(s);
+    plan->small_tiles += tiles_of(s);
     cur.y++;
     cur.z += slots_of(s);
     cur.w += tiles_of(s);
@@ -1031,15 +1033,39 @@ void Synthesis::buildUnits() {
     throw Error(SB_ERR_UNSUPPORTED, "too many tiles on the fused path");
   }
   fused_tiles = static_cast<int>(ftiles);
-  const int slots_cap = (opt.max_atoms_per_unit > 0) ? opt.max_atoms_per_unit : 256;
-  // Default packing: molecules of four or fewer tiles share a unit, larger ones run alone
-  // (measured on 1,024 molecules of 16-256 atoms: 213 us against 238 us for units packed up to
-  // 36 tiles, which leave a sliver of a second wave)
-  const int tiles_cap = (opt.max_tiles_per_unit > 0) ? opt.max_tiles_per_unit : 4;
+  int nfused = 0, widest = 0;   // molecules on the fused path, atom slots of the largest
+  for (int s = 0; s < nsys; s++) {
+    if (tiled_index[s] < 0) {
+      nfused++;
+      widest = std::max(widest, (atom_count[s] + kTile - 1) / kTile * kTile);
+    }
+  }
+  // Default packing.  Molecules of more than 128 atoms among them: molecules of four or fewer tiles
+  // share a unit, larger ones run alone (1,024 molecules of 16-256 atoms: 213 us against 238 us for
+  // units packed up to 36 tiles, which leave a sliver of a second wave).  All molecules of up to
+  // 128 atoms: one a unit while that is one wave of 256-thread blocks (512 molecules of 24-96 atoms
+  // 44 us, four tiles a unit 52), and again beyond 1.25 waves, where launchThreads() takes 128-thread
+  // blocks (1,024 molecules: 71 us, four tiles a unit in 256-thread blocks 81); from two waves of
+  // those on, units of up to eight tiles if the molecules average fewer than five (4,096 molecules:
+  // 253 us, one a unit 260, four tiles a unit in 256-thread blocks 293).
+  int slots_cap = 256, tiles_cap = 4;
+  if (widest <= 128 && nfused <= 4 * sm_count) {
+    tiles_cap = 1;
+  }
+  else if (widest <= 128 && nfused > 5 * sm_count) {
+    slots_cap = 128;
+    tiles_cap = (nfused > 16 * sm_count && ftiles < 5LL * nfused) ? 8 : 1;
+  }
+  if (opt.max_atoms_per_unit > 0) slots_cap = opt.max_atoms_per_unit;
+  if (opt.max_tiles_per_unit > 0) tiles_cap = opt.max_tiles_per_unit;
   eval_plan = makePlan(slots_cap, tiles_cap, true);
-  // minimization keeps whole molecules on chip for hundreds of cycles: smaller units balance
-  // the persistent grid better (sb_autotune can choose another packing)
-  min_plan = makePlan(128, 16, true);
+  // Minimization keeps whole molecules on chip for hundreds of cycles.  A batch of at most one
+  // molecule per SM gives each its own block, in one launch and with 512 threads (launchMinPlan):
+  // such a launch lasts as long as its largest molecule.  128 molecules of 12-512 atoms, 60 cycles:
+  // one launch after another with 256 threads 16.8 ms, this way 8.2 ms.  Larger batches share units of up to 128 slots, which balance the persistent grid
+  // (sb_autotune can choose another packing).
+  min_plan = (nfused <= sm_count) ? makePlan(std::max(widest, kTile), 1, true) :
+                                    makePlan(128, 16, true);
   // one unit per system, in system order, for the per-system launches
   auto slots_of = [&](int s) { return (atom_count[s] + kTile - 1) / kTile * kTile; };
   auto tiles_of = [&](int s) {
@@ -1321,29 +1347,42 @@ void Synthesis::launchPlan(const UnitPlan &plan, int terms, bool force, bool ene
   if (plan.n_big > 0) {
     d.max_unit_slots = plan.big_slots;
     cudaCheck(launchEvalFused(d, 0, plan.n_big, plan.big_lj, terms, force, energy, plan.n_big,
-                              launchThreads(plan.n_big, terms), stream, clash.on()),
+                              launchThreads(plan.n_big, plan.big_slots, plan.big_tiles, terms),
+                              stream, clash.on()),
               "fused evaluation launch (large molecules)");
   }
   if (nunit > plan.n_big) {
     d.max_unit_slots = plan.small_slots;
     cudaCheck(launchEvalFused(d, plan.n_big, nunit, plan.small_lj, terms, force, energy,
-                              nunit - plan.n_big, launchThreads(nunit - plan.n_big, terms),
-                              stream, clash.on()),
+                              nunit - plan.n_big,
+                              launchThreads(nunit - plan.n_big, plan.small_slots,
+                                            plan.small_tiles, terms), stream, clash.on()),
               "fused evaluation launch");
   }
 }
 
-// Threads a block for an evaluation launch of `units` work units: the configured count, or
-// 512 when the launch evaluates every term and its units fit in one wave of 256-thread blocks
-// (four an SM), where twice the warps on each unit finish the wave sooner (475 units of 16-256
-// atoms: 141 us against 184); beyond one wave the 256-thread blocks are faster.  Sums are
-// fixed-point, so the block size changes no result bit.
-int Synthesis::launchThreads(int units, int terms) const {
-  if (opt.threads_per_block > 0 || !allow_wide || terms != SB_TERM_ALL ||
-      units >= 4 * sm_count) {
+// Threads a block for an evaluation launch of `units` work units of up to `slots` atom slots and
+// `tiles` tiles in all: the configured count, or
+//   128 when the units are small (up to 128 slots) and more than 1.25 waves of 256-thread blocks:
+//       eight blocks an SM, whose four warps the few tiles of a unit keep busy (4,096 molecules of
+//       24-96 atoms: 253 us against 263 for the same units in 256-thread blocks, energies alone 127
+//       against 145; 1,024: 71 against 75);
+//   512 when the launch evaluates every term and all its units are resident at two such blocks an
+//       SM, or its units average eight tiles and fit in one wave of 256-thread blocks (336 units of
+//       20-200 atoms: 70 us against 93; but 545 units of 24-96 atoms 64 against 48).
+// Sums are fixed-point, so the block size changes no result bit.
+int Synthesis::launchThreads(int units, int slots, long long tiles, int terms) const {
+  if (opt.threads_per_block > 0 || !allow_wide) {
     return threads;
   }
-  return 512;
+  if (slots <= 128 && units > 5 * sm_count) {
+    return 128;
+  }
+  if (terms == SB_TERM_ALL &&
+      (units <= 2 * sm_count || (units < 4 * sm_count && tiles >= 8LL * units))) {
+    return 512;
+  }
+  return threads;
 }
 
 void Synthesis::evaluate(int terms, bool force, bool energy, cudaStream_t stream,
@@ -1826,6 +1865,12 @@ void Synthesis::graphFinalEnergy(int first, int count, bool single, cudaStream_t
   cudaCheck(launchLineStep(dev, dev_min, first, count, 4, stream), "line search launch");
 }
 
+void Synthesis::checkMinimizeSmem(int slots, int lj) const {
+  if (static_cast<int>(minimizeSmemBytes(slots, lj)) > max_smem_optin) {
+    throw Error(SB_ERR_UNSUPPORTED, "a molecule is too large for on-chip minimization");
+  }
+}
+
 void Synthesis::launchMinPlan(const UnitPlan &plan, int cycles, bool final_energy,
                               cudaStream_t stream) {
   DevMinimizer m = dev_min;
@@ -1838,17 +1883,18 @@ void Synthesis::launchMinPlan(const UnitPlan &plan, int cycles, bool final_energ
   if (plan.n_big > 0) {
     d.max_unit_slots = plan.big_slots;
     m.queue = d_queue.p;
-    if (static_cast<int>(minimizeSmemBytes(plan.big_slots, plan.big_lj)) > max_smem_optin) {
-      throw Error(SB_ERR_UNSUPPORTED, "a molecule is too large for on-chip minimization");
-    }
+    checkMinimizeSmem(plan.big_slots, plan.big_lj);
     cudaCheck(launchMinimize(d, m, 0, plan.n_big, plan.big_lj, cycles, final_energy, threads,
                              sm_count, stream), "minimization launch (large molecules)");
   }
   if (nunit > plan.n_big) {
     d.max_unit_slots = plan.small_slots;
     m.queue = d_queue.p + 1;
+    checkMinimizeSmem(plan.small_slots, plan.small_lj);
+    // a block per SM at most: twice the warps on each unit
+    const int wide = (opt.threads_per_block <= 0 && nunit - plan.n_big <= sm_count) ? 512 : threads;
     cudaCheck(launchMinimize(d, m, plan.n_big, nunit, plan.small_lj, cycles, final_energy,
-                             threads, sm_count, stream), "minimization launch");
+                             wide, sm_count, stream), "minimization launch");
   }
 }
 
@@ -1954,9 +2000,7 @@ void Synthesis::minimizeRange(int first, int count, const sb_minimize_controls &
   d.unit_meta = single_plan->d_meta.p;
   d.nunit = nsys;
   d.max_unit_slots = single_slots;
-  if (static_cast<int>(minimizeSmemBytes(single_slots, single_lj)) > max_smem_optin) {
-    throw Error(SB_ERR_UNSUPPORTED, "a molecule is too large for on-chip minimization");
-  }
+  checkMinimizeSmem(single_slots, single_lj);
   // one block per launch: the unit counter is never consulted for a second unit
   for (int s = first; s < first + count; s++) {
     cudaCheck(launchMinimize(d, dev_min, s, s + 1, single_lj, ctl.total_cycles, true, threads,
@@ -2411,9 +2455,12 @@ int sb_launch_info(const sb_synthesis* syn, int* work_units, int* blocks, int* t
     if (blocks) *blocks = s->eval_plan->units.size();
     if (threads) {
       // block size of the batched evaluation's launch of packed units
-      const int n = static_cast<int>(s->eval_plan->units.size());
-      const int packed = n - s->eval_plan->n_big;
-      *threads = s->launchThreads(packed > 0 ? packed : n, SB_TERM_ALL);
+      const sb::UnitPlan &plan = *s->eval_plan;
+      const int n = static_cast<int>(plan.units.size());
+      const int packed = n - plan.n_big;
+      *threads = (packed > 0) ? s->launchThreads(packed, plan.small_slots, plan.small_tiles,
+                                                 SB_TERM_ALL) :
+                                s->launchThreads(n, plan.big_slots, plan.big_tiles, SB_TERM_ALL);
     }
   });
 }

@@ -164,6 +164,7 @@ struct UnitPlan {
   int n_big = 0;                 // units [0, n_big) hold one molecule above the packing cap
   int big_slots = 0, big_lj = 0;
   int small_slots = 0, small_lj = 0;
+  long long big_tiles = 0, small_tiles = 0;
   std::vector<int> meta;         // kUnitMetaFields ints per molecule row, plus a closing row
   std::vector<int4> desc;        // as units, but x = first row of the unit in meta
   DeviceArray<int4> d_units;     // desc on the device
@@ -209,7 +210,7 @@ public:
   std::vector<double> h_sasa_radius;   // per padded atom: half the LJ sigma of (type 0, type)
   void downloadResults(double* forces, double* energies, cudaStream_t stream);
   void setRestraints(const sb_restraint* list, int count);
-  int launchThreads(int units, int terms) const;
+  int launchThreads(int units, int slots, long long tiles, int terms) const;
   void getEnergiesFixed(long long* out, cudaStream_t stream);
   void getGbWorkspace(double* psi, double* radii, double* sde, cudaStream_t stream);
   int checkStatus(cudaStream_t stream);
@@ -382,6 +383,7 @@ private:
   bool allow_wide = true;        // 512-thread blocks for small all-term launches (autotuned)
   void launchPlan(const UnitPlan &plan, int terms, bool force, bool energy, cudaStream_t stream,
                   const Clash &clash = Clash());
+  void checkMinimizeSmem(int slots, int lj) const;
   void launchMinPlan(const UnitPlan &plan, int cycles, bool final_energy, cudaStream_t stream);
   void launchTiledRange(int mol_begin, int mol_end, int terms, bool force, bool energy,
                         cudaStream_t stream, const Clash &clash = Clash());

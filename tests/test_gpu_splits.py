@@ -24,3 +24,46 @@ def test_tile_runs_change_no_bit(precision):
         assert np.array_equal(fa, fb[k])
     alone.close()
     batch.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("count,threads", [(296, 512), (300, 256), (592, 256), (760, 128),
+                                           (2400, 128)])
+def test_packing_and_block_size_rules_change_no_bit(count, threads):
+    """The default packing and block size of batches of small molecules on both sides of each
+    line (148 SMs), against one molecule a unit in 256-thread blocks."""
+    import stormm_b200 as sb
+    from stormm_b200 import synthetic
+    mols = [synthetic.make_molecule(700 + k, n) for k, n in enumerate((17, 24, 33, 47, 64, 96))]
+    index = np.arange(count, dtype=np.int32) % len(mols)
+    xyz = np.concatenate([mols[t].coords for t in index])
+    syns = [sb.Synthesis(mols, topology_index=index),
+            sb.Synthesis(mols, topology_index=index, threads_per_block=256, max_tiles_per_unit=1)]
+    assert syns[0].launch_info()["threads"] == threads
+    out = []
+    for syn in syns:
+        syn.set_coordinates(xyz)
+        syn.initialize()
+        syn.evaluate()
+        out.append((syn.energies_fixed(), syn.forces_fixed()[0]))
+        syn.close()
+    assert np.array_equal(out[0][0], out[1][0])
+    assert np.array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.gpu
+def test_on_chip_minimizer_block_size_changes_no_bit():
+    """148 molecules take a 512-thread block each, 149 share units of 256-thread blocks."""
+    import stormm_b200 as sb
+    from stormm_b200 import synthetic
+    mols = [synthetic.make_molecule(800 + k, n) for k, n in enumerate((20, 40, 130, 300))]
+    final = []
+    for count in (148, 149):
+        index = np.arange(count, dtype=np.int32) % len(mols)
+        syn = sb.Synthesis(mols, topology_index=index)
+        syn.set_coordinates(np.concatenate([mols[t].coords for t in index]))
+        syn.minimize(total_cycles=12, sd_cycles=4, kernel=sb.MIN_PERSISTENT)
+        final.append(syn.split(syn.coordinates())[:148])
+        syn.close()
+    for a, b in zip(*final):
+        assert np.array_equal(a, b)
