@@ -9,6 +9,12 @@
 // formats, psi and dE/dR at 2^40 (finer than the FP32 path's, so the integer grid does not limit
 // the FP64 result), hence results are bit-identical run to run.  Valence terms are one thread per
 // term (Potential/valence_potential.tpp:9-578, 1288-1420).
+//
+// The passes are bound by FP64 issue (two cycles a warp instruction), so divisions and square roots
+// are taken through rsqrt() and stored reciprocals, whose errors of an ulp or two are far below the
+// grids the sums are kept on, and pass 1 sets near pairs aside.  Against sqrt() and divisions per
+// pair and closed forms on a branch: 128 molecules of 16-256 atoms, force + energy with copies,
+// 276 -> 206 us; 8 chains of 2,000-5,000 atoms 1,848 -> 1,308 us; same error against 64 bits.
 #include <cuda_runtime.h>
 
 #include "stormm_b200.h"
@@ -97,35 +103,41 @@ __device__ __forceinline__ void warpEnergy64(const DevSynthesis &d, int sysid, i
 // ------------------------------------------------------------------------------------------------
 // HCT descreening and its radial derivative, the reference's case by case forms
 // ------------------------------------------------------------------------------------------------
-__device__ __forceinline__ double hctIntegral64(double r, double rho, double sj) {
-  const double r2 = r * r;
-  const double invr = 1.0 / r;
+// At distance r (r2 = r^2, invr = 1 / r) of an atom of offset radius rho (inv_rho = 1 / rho) by a
+// neighbour of screened radius sj.  Reciprocals are shared between terms: (r - sj) / (r + sj) is
+// (r - sj)^2 / (r^2 - sj^2).
+// The far form alone (r > 4 sj)
+__device__ __forceinline__ double hctFar64(double invr2, double sj) {
+  const double t = sj * sj * invr2;
+  return sj * t * invr2 *
+         (kTaylorA64 + t * (kTaylorB64 + t * (kTaylorC64 + t * (kTaylorD64 + t * kTaylorDD64))));
+}
+
+__device__ __forceinline__ double hctIntegral64(double r, double r2, double invr, double rho,
+                                                double inv_rho, double sj) {
   const double sj2 = sj * sj;
   if (r > 4.0 * sj) {
-    const double invr2 = invr * invr;
-    const double t = sj2 * invr2;
-    return sj * t * invr2 *
-           (kTaylorA64 + t * (kTaylorB64 + t * (kTaylorC64 + t * (kTaylorD64 + t * kTaylorDD64))));
+    return hctFar64(invr * invr, sj);
   }
-  if (r > rho + sj) {
-    return 0.5 * (sj / (r2 - sj2) + 0.5 * invr * log((r - sj) / (r + sj)));
+  const bool apart = r > rho + sj;
+  const bool part = !apart && r > fabs(rho - sj);
+  if (!apart && !part && !(rho < sj)) {
+    return 0.0;
   }
-  if (r > fabs(rho - sj)) {
-    const double inv_rho = 1.0 / rho;
+  // 1 / (r^2 - sj^2) without overlap or inside the neighbour, 1 / (r + sj) on partial overlap
+  const double den = 1.0 / (part ? r + sj : r2 - sj2);
+  const double d = r - sj;
+  const double lg = log(part ? rho * den : (apart ? d * d * den : -d * d * den));
+  if (part) {
     const double theta = 0.5 * inv_rho * invr * (r2 + rho * rho - sj2);
-    const double uij = 1.0 / (r + sj);
-    return 0.25 * (inv_rho * (2.0 - theta) - uij + invr * log(rho * uij));
+    return 0.25 * (inv_rho * (2.0 - theta) - den + invr * lg);
   }
-  if (rho < sj) {
-    return 0.5 * (sj / (r2 - sj2) + 2.0 / rho + 0.5 * invr * log((sj - r) / (sj + r)));
-  }
-  return 0.0;
+  return 0.5 * (sj * den + (apart ? 0.0 : 2.0 * inv_rho) + 0.5 * invr * lg);
 }
 
 // -(1/r) dI/dr
-__device__ __forceinline__ double hctDerivative64(double r, double rho, double sj) {
-  const double r2 = r * r;
-  const double invr = 1.0 / r;
+__device__ __forceinline__ double hctDerivative64(double r, double r2, double invr, double rho,
+                                                  double inv_rho, double sj) {
   const double invr2 = invr * invr;
   const double sj2 = sj * sj;
   if (r > 4.0 * sj) {
@@ -133,23 +145,20 @@ __device__ __forceinline__ double hctDerivative64(double r, double rho, double s
     return t * sj * invr2 * invr2 *
            (kTaylorE64 + t * (kTaylorF64 + t * (kTaylorG64 + t * (kTaylorH64 + t * kTaylorHH64))));
   }
-  if (r > rho + sj) {
-    const double temp1 = 1.0 / (r2 - sj2);
-    return temp1 * sj * (-0.5 * invr2 + temp1) + 0.25 * invr * invr2 * log((r - sj) / (r + sj));
+  const bool apart = r > rho + sj;
+  const bool part = !apart && r > fabs(rho - sj);
+  if (!apart && !part && !(rho < sj)) {
+    return 0.0;
   }
-  if (r > fabs(rho - sj)) {
-    const double temp1 = 1.0 / (r + sj);
-    const double invr3 = invr2 * invr;
-    const double inv_rho = 1.0 / rho;
+  const double den = 1.0 / (part ? r + sj : r2 - sj2);
+  const double d = r - sj;
+  const double lg = log(part ? rho * den : (apart ? d * d * den : -d * d * den));
+  const double invr3 = invr2 * invr;
+  if (part) {
     return -0.25 * (-0.5 * (r2 - rho * rho + sj2) * invr3 * inv_rho * inv_rho +
-                    invr * temp1 * (temp1 - invr) - invr3 * log(rho * temp1));
+                    invr * den * (den - invr) - invr3 * lg);
   }
-  if (rho < sj) {
-    const double temp1 = 1.0 / (r2 - sj2);
-    return -0.5 * (sj * invr2 * temp1 - 2.0 * sj * temp1 * temp1 -
-                   0.5 * invr2 * invr * log((sj - r) / (sj + r)));
-  }
-  return 0.0;
+  return den * sj * (den - 0.5 * invr2) + 0.25 * invr3 * lg;
 }
 
 // Run one tile: p.pair(jslot, jl) for every pair of the tile (once each) and p.rotate() after
@@ -188,40 +197,78 @@ __device__ __forceinline__ int traveledAtom(const TileInfo &ti, int lane) {
 // ------------------------------------------------------------------------------------------------
 // Pair functors for walkTile64
 // ------------------------------------------------------------------------------------------------
-// Pass 1 payload: w1 = s * rho, w2 = rho, code = neck index
+// Pass 1 payload: w1 = s * rho, w2 = rho, w3 = 1 / rho, code = neck index.  The walk takes the far
+// form for every pair; the pairs with r <= 4 sj in either direction, which a small molecule has on
+// some lane at almost every step, are marked by their step in `late` and evaluated densely after it
+// (spreadLate), a closed form costing a division and a logarithm.
 struct Radii64 {
   Stage64 v;
   Neck64 neck;
   double4 ai, bi;
   int ni;
   double psi_i, psi_j;
+  unsigned late, bit;
   __device__ Radii64(const Stage64 &v_in, const Neck64 &n) : v(v_in), neck(n) {}
-  __device__ __forceinline__ void begin(int islot) {
+  __device__ __forceinline__ void begin(int islot, bool diag) {
     ai = v.pa[islot];
     bi = v.pb[islot];
     ni = v.code[islot];
     psi_i = psi_j = 0.0;
+    late = 0u;
+    bit = diag ? 2u : 1u;
   }
   __device__ __forceinline__ void pair(int jslot, int) {
     const double4 aj = v.pa[jslot];
-    const double4 bj = v.pb[jslot];
     const double dx = aj.x - ai.x, dy = aj.y - ai.y, dz = aj.z - ai.z;
-    const double r = sqrt(dx * dx + dy * dy + dz * dz);
-    psi_i -= hctIntegral64(r, bi.x, aj.w);
-    psi_j -= hctIntegral64(r, bj.x, ai.w);
-    if (neck.size > 0 && r < bi.x + bj.x + neck.reach) {
-      const int nj = v.code[jslot];
-      double unused;
-      psi_i -= neck.term(ni, nj, r, &unused);
-      psi_j -= neck.term(nj, ni, r, &unused);
+    const double r2 = dx * dx + dy * dy + dz * dz;
+    const double invr = rsqrt(r2);
+    const double r = r2 * invr;
+    const double invr2 = invr * invr;
+    const bool later = !(r > 4.0 * aj.w && r > 4.0 * ai.w);
+    const double hi = hctFar64(invr2, aj.w), hj = hctFar64(invr2, ai.w);
+    late |= later ? bit : 0u;
+    psi_i -= later ? 0.0 : hi;
+    psi_j -= later ? 0.0 : hj;
+    if (neck.size > 0 && !later) {
+      const double rho_j = v.pb[jslot].x;
+      if (r < bi.x + rho_j + neck.reach) {
+        const int nj = v.code[jslot];
+        double unused;
+        psi_i -= neck.term(ni, nj, r, &unused);
+        psi_j -= neck.term(nj, ni, r, &unused);
+      }
     }
   }
   __device__ __forceinline__ void rotate(int lane) {
     psi_j = __shfl_sync(0xffffffffu, psi_j, (lane + 1) & 31);
+    bit <<= 1;
+  }
+  // The pairs left out; add(slot, v) adds v to a slot's descreening sum
+  template <class Add>
+  __device__ __forceinline__ void finish(const TileInfo &ti, int lane, unsigned short* list,
+                                         const Add &add) const {
+    spreadLate(late, list, lane, [&](int of, int k) {
+      const int is = ti.ibase + of, js = ti.jbase + ((of + k) & 31);
+      const double4 a = v.pa[is], c = v.pa[js];
+      const double4 b = v.pb[is], d = v.pb[js];
+      const double dx = c.x - a.x, dy = c.y - a.y, dz = c.z - a.z;
+      const double r2 = dx * dx + dy * dy + dz * dz;
+      const double invr = rsqrt(r2);
+      const double r = r2 * invr;
+      double hi = hctIntegral64(r, r2, invr, b.x, b.z, c.w);
+      double hj = hctIntegral64(r, r2, invr, d.x, d.z, a.w);
+      if (neck.size > 0 && r < b.x + d.x + neck.reach) {
+        double unused;
+        hi += neck.term(v.code[is], v.code[js], r, &unused);
+        hj += neck.term(v.code[js], v.code[is], r, &unused);
+      }
+      add(is, -hi);
+      add(js, -hj);
+    });
   }
 };
 
-// Pass 2 payload: w1 = charge x sqrt(Coulomb constant), w2 = effective radius
+// Pass 2 payload: w1 = charge x sqrt(Coulomb constant), w2 = effective radius, w3 = 1 / w2
 // Softened cores in FP64 (STORMM's Potential/soft_core_potentials.tpp, the FP32 path's
 // softCorePair in double): the clash distance and sigma ratio of a system, scaled by its
 // minimization progress when a cycle count is given
@@ -270,7 +317,7 @@ struct Pair64 {
     const double qiqj = ai.w * aj.w;
     double fmag = 0.0;
     if (NB && CLASH && ((mask >> jl) & 1u) == 0u && (cl.x > 0.0 || cl.y > 0.0)) {
-      const double invr = 1.0 / sqrt(r2);
+      const double invr = rsqrt(r2);
       const double2 ab = lj[code_i + v.code[jslot]];
       double ee = 0.0, ev = 0.0;
       fmag = softCorePair64(r2 * invr, invr, qiqj, ab.x, ab.y, cl.x, qc, cl.y, &ee, &ev);
@@ -283,8 +330,8 @@ struct Pair64 {
       }
     }
     else if (NB && ((mask >> jl) & 1u) == 0u) {
-      const double invr2 = 1.0 / r2;
-      const double invr = sqrt(invr2);
+      const double invr = rsqrt(r2);
+      const double invr2 = invr * invr;
       const double invr4 = invr2 * invr2;
       const double2 ab = lj[code_i + v.code[jslot]];
       if (ENERGY) {
@@ -298,10 +345,14 @@ struct Pair64 {
     if (GB) {
       // nonbonded_potential.tpp:880-920
       const double ijb = bi.x * bj.x;
-      const double efac = exp(-r2 / (4.0 * ijb));
-      const double fgbi = 1.0 / sqrt(r2 + ijb * efac);
-      const double fgbk = -kappa * kGbKscale64 / fgbi;
-      const double expmkf = ((kappa > 0.0) ? exp(fgbk) : 1.0) * inv_diel;
+      const double efac = exp(-0.25 * r2 * bi.z * bj.z);
+      const double f2gb = r2 + ijb * efac;
+      const double fgbi = rsqrt(f2gb);
+      double fgbk = 0.0, expmkf = inv_diel;
+      if (kappa > 0.0) {
+        fgbk = -kappa * kGbKscale64 * f2gb * fgbi;
+        expmkf = exp(fgbk) * inv_diel;
+      }
       const double dielfac = 1.0 - expmkf;
       if (ENERGY) {
         e_gb -= qiqj * dielfac * fgbi;
@@ -336,8 +387,8 @@ struct Pair64 {
   }
 };
 
-// Pass 3 payload: w1 = s * rho, w2 = rho, w3 = dE/dR after the chain-rule prefactor, code = neck
-// index
+// Pass 3 payload: w1 = s * rho, w2 = rho, w3 = 1 / rho, w4 = dE/dR after the chain-rule prefactor,
+// code = neck index
 struct Deriv64 {
   Stage64 v;
   Neck64 neck;
@@ -355,14 +406,17 @@ struct Deriv64 {
     const double4 aj = v.pa[jslot];
     const double4 bj = v.pb[jslot];
     const double dx = aj.x - ai.x, dy = aj.y - ai.y, dz = aj.z - ai.z;
-    const double r = sqrt(dx * dx + dy * dy + dz * dz);
-    double fmag = hctDerivative64(r, bi.x, aj.w) * bi.y + hctDerivative64(r, bj.x, ai.w) * bj.y;
+    const double r2 = dx * dx + dy * dy + dz * dz;
+    const double invr = rsqrt(r2);
+    const double r = r2 * invr;
+    double fmag = hctDerivative64(r, r2, invr, bi.x, bi.z, aj.w) * bi.w +
+                  hctDerivative64(r, r2, invr, bj.x, bj.z, ai.w) * bj.w;
     if (neck.size > 0 && r < bi.x + bj.x + neck.reach) {
       const int nj = v.code[jslot];
       double dij, dji;
       neck.term(ni, nj, r, &dij);
       neck.term(nj, ni, r, &dji);
-      fmag += dij * bi.y + dji * bj.y;
+      fmag += dij * bi.w + dji * bj.w;
     }
     fxi -= fmag * dx;
     fyi -= fmag * dy;
@@ -406,18 +460,20 @@ __device__ __forceinline__ void stageTile64(const DevSynthesis &d, const DevPrec
       if (PASS == 2) {
         pa.w = p.charge[gi];
         pb.x = p.radius[gi];
+        pb.z = 1.0 / pb.x;
       }
       else {
         pa.w = p.srho[gi];
         pb.x = p.rho[gi];
+        pb.z = 1.0 / pb.x;
         if (PASS == 3) {
-          pb.y = p.sde[gi];
+          pb.w = p.sde[gi];
         }
       }
     }
     else {
       pa = make_double4(5000.0 + 16.0 * static_cast<double>(slot), 0.0, 0.0, 0.0);
-      pb = make_double4(1.0, 0.0, 0.0, 0.0);
+      pb = make_double4(1.0, 0.0, 1.0, 0.0);
     }
     v.pa[slot] = pa;
     v.pb[slot] = pb;
@@ -426,11 +482,12 @@ __device__ __forceinline__ void stageTile64(const DevSynthesis &d, const DevPrec
   __syncwarp();
 }
 
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 3)
 kRadii64(const DevSynthesis d, const DevPrecise p, const DevTiled t, int tile_begin,
          int tile_end) {
   __shared__ double4 pa[kTiledWarps * kSlots64], pb[kTiledWarps * kSlots64];
   __shared__ int code[kTiledWarps * kSlots64];
+  __shared__ unsigned short lists[kTiledWarps][kLateEntries];
   const int lane = threadIdx.x & 31;
   int first, last;
   warpTileRange(t, tile_begin, tile_end, &first, &last);
@@ -442,16 +499,19 @@ kRadii64(const DevSynthesis d, const DevPrecise p, const DevTiled t, int tile_be
     int I, J;
     const TileInfo ti = tiledTileInfo(d, sysid, g - t.tile_prefix[m], &I, &J);
     stageTile64<1>(d, p, t, v, sysid, I, J, ti.diag, lane);
-    f.begin(lane);
+    f.begin(lane, ti.diag);
     walkTile64(f, ti, lane);
-    const int base = d.atom_start[sysid];
+    const int ia = d.atom_start[sysid] + I * kTile, ja = d.atom_start[sysid] + J * kTile;
     if (lane < ti.ni) {
-      addFixed(&t.psi_acc[base + I * kTile + lane], f.psi_i * kAcc64Scale);
+      addFixed(&t.psi_acc[ia + lane], f.psi_i * kAcc64Scale);
     }
     const int jl = traveledAtom(ti, lane);
     if (jl < ti.nj) {
-      addFixed(&t.psi_acc[base + J * kTile + jl], f.psi_j * kAcc64Scale);
+      addFixed(&t.psi_acc[ja + jl], f.psi_j * kAcc64Scale);
     }
+    f.finish(ti, lane, lists[threadIdx.x >> 5], [&](int slot, double x) {
+      addFixed(&t.psi_acc[slot < kTile ? ia + slot : ja + slot - kTile], x * kAcc64Scale);
+    });
     __syncwarp();
   }
 }
@@ -523,7 +583,7 @@ kPair64(const DevSynthesis d, const DevPrecise p, const DevTiled t, int tile_beg
   }
 }
 
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 3)
 kDeriv64(const DevSynthesis d, const DevPrecise p, const DevTiled t, int tile_begin,
          int tile_end) {
   __shared__ double4 pa[kTiledWarps * kSlots64], pb[kTiledWarps * kSlots64];
@@ -698,12 +758,14 @@ template <bool FORCE, bool ENERGY, bool CLASH>
 __global__ void __launch_bounds__(256)
 kValence64(const DevSynthesis d, const DevPrecise p, const DevTiled t, int mol_begin,
            int mol_end) {
+  // one kind of term per block row, so that the three run side by side
+  const int kind = blockIdx.y;
   const int stride = gridDim.x * blockDim.x;
   const int first_sys = t.systems[mol_begin];
   const int last_sys = t.systems[mol_end - 1];
   // harmonic bonds, valence_potential.tpp:9-97
   for (int k = d.bond_start[first_sys] + blockIdx.x * blockDim.x + threadIdx.x;
-       k < d.bond_start[last_sys + 1]; k += stride) {
+       kind == kBondTerms && k < d.bond_start[last_sys + 1]; k += stride) {
     const int sysid = termOwner(d.bond_start, d.nsys, k);
     const Atoms64 at{d, d.atom_start[sysid]};
     const int2 ij = p.bond_atoms[k];
@@ -722,7 +784,7 @@ kValence64(const DevSynthesis d, const DevPrecise p, const DevTiled t, int mol_b
   }
   // harmonic angles, valence_potential.tpp:170-288
   for (int k = d.angl_start[first_sys] + blockIdx.x * blockDim.x + threadIdx.x;
-       k < d.angl_start[last_sys + 1]; k += stride) {
+       kind == kAnglTerms && k < d.angl_start[last_sys + 1]; k += stride) {
     const int sysid = termOwner(d.angl_start, d.nsys, k);
     const Atoms64 at{d, d.atom_start[sysid]};
     const int4 ijk = p.angl_atoms[k];
@@ -756,7 +818,7 @@ kValence64(const DevSynthesis d, const DevPrecise p, const DevTiled t, int mol_b
   }
   // cosine dihedrals with attached 1-4 pairs, valence_potential.tpp:359-578, 1288-1420
   for (int k = d.dihe_start[first_sys] + blockIdx.x * blockDim.x + threadIdx.x;
-       k < d.dihe_start[last_sys + 1]; k += stride) {
+       kind == kDiheTerms && k < d.dihe_start[last_sys + 1]; k += stride) {
     const int sysid = termOwner(d.dihe_start, d.nsys, k);
     const Atoms64 at{d, d.atom_start[sysid]};
     const int4 ijkl = p.dihe_atoms[k];
@@ -885,7 +947,7 @@ cudaError_t launchTiled64(const DevSynthesis &d, const DevPrecise &p, const DevT
   const int tgrid = tileGrid(te - tb, sm_count);
   const int agrid = atomGrid(ae - ab, sm_count);
   if (vale) {
-    const int vgrid = sm_count * 4;
+    const dim3 vgrid(sm_count * 2, 3);
 #define SB_VALE64(C)                                                                            \
     if (force && energy) kValence64<true, true, C><<<vgrid, 256, 0, stream>>>(d, p, t, mol_begin, mol_end); \
     else if (force) kValence64<true, false, C><<<vgrid, 256, 0, stream>>>(d, p, t, mol_begin, mol_end);    \

@@ -44,12 +44,12 @@ def test_block_edges_match_the_oracle(route):
     syn.close()
 
 
-@pytest.mark.parametrize("route", ["fused", "tiled"])
+@pytest.mark.parametrize("route", ["fused", "tiled", "fp64"])
 @pytest.mark.parametrize("natom,scale", [(16, 0.2), (40, 0.25), (64, 0.15), (97, 0.3)])
 def test_overlapping_pairs_beyond_the_list(route, natom, scale):
     m = copy.deepcopy(synthetic.make_molecule(4100 + natom, natom))
     m.coords = m.coords * scale
-    opts = dict(tiled_above_atoms=32) if route == "tiled" else {}
+    opts = {"fused": {}, "tiled": dict(tiled_above_atoms=32), "fp64": dict(precision=1)}[route]
     ref = oracle.from_molecule(m).evaluate(m.coords)
     syn = sb.Synthesis([m], **opts)
     syn.set_coordinates(m.coords)
