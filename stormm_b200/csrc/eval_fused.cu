@@ -93,10 +93,10 @@ kEvalFused(const DevSynthesis d, int unit_begin, int unit_end, int max_lj) {
   evalFusedUnits<FORCE, ENERGY, TERMS, CLASH, NECK>(d, unit_begin, unit_end, max_lj);
 }
 
-// The same with 512 threads a block: twice the warps per work unit, for launches of too few
+// The same with 512 or 1,024 threads a block: more warps per work unit, for launches of too few
 // units to fill the GPU with 256-thread blocks (a small batch, or its large molecules)
-template <bool FORCE, bool ENERGY, int TERMS, bool CLASH, bool NECK>
-__global__ void __launch_bounds__(512, 2)
+template <bool FORCE, bool ENERGY, int TERMS, bool CLASH, bool NECK, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1024 / THREADS)
 kEvalFusedWide(const DevSynthesis d, int unit_begin, int unit_end, int max_lj) {
   evalFusedUnits<FORCE, ENERGY, TERMS, CLASH, NECK>(d, unit_begin, unit_end, max_lj);
 }
@@ -109,17 +109,18 @@ cudaError_t launchEvalFused(const DevSynthesis &d, int unit_begin, int unit_end,
   // softened cores change only Coulomb, Lennard-Jones and 1-4 terms, the neck term only GB
   clash = clash && (terms & 3) != 0;
   const bool neck = d.neck_size > 0 && (terms & 4) != 0;
-  // 512-thread blocks exist for evaluations of all terms only
+  // blocks of more than 256 threads exist for evaluations of all terms only
   if (threads > 256 && terms != 7) {
     threads = 256;
   }
-  if (threads != 512 && (threads < 64 || threads > 256 || threads % 32 != 0)) {
+  if (threads != 512 && threads != 1024 && (threads < 64 || threads > 256 || threads % 32 != 0)) {
     return cudaErrorInvalidValue;
   }
-#define SB_PICK(K, F, E, T)                                                                     \
-    (neck ? (clash ? K<F, E, T, ((T) & 3) != 0, ((T) & 4) != 0> :                               \
-                     K<F, E, T, false, ((T) & 4) != 0>) :                                       \
-            (clash ? K<F, E, T, ((T) & 3) != 0, false> : K<F, E, T, false, false>))
+#define SB_PICK(K, F, E, T, ...)                                                                \
+    (neck ? (clash ? K<F, E, T, ((T) & 3) != 0, ((T) & 4) != 0 __VA_ARGS__> :                   \
+                     K<F, E, T, false, ((T) & 4) != 0 __VA_ARGS__>) :                           \
+            (clash ? K<F, E, T, ((T) & 3) != 0, false __VA_ARGS__> :                            \
+                     K<F, E, T, false, false __VA_ARGS__>))
 #define SB_GO(KERN)                                                                             \
   {                                                                                             \
     auto kern = KERN;                                                                           \
@@ -128,12 +129,14 @@ cudaError_t launchEvalFused(const DevSynthesis &d, int unit_begin, int unit_end,
     kern<<<blocks, threads, smem, stream>>>(d, unit_begin, unit_end, max_lj);                   \
     return cudaGetLastError();                                                                  \
   }
+#define SB_COMMA ,
 #define SB_LAUNCH(F, E, T)                                                                      \
   {                                                                                             \
     if constexpr ((T) == 7) {                                                                   \
-      if (threads > 256) SB_GO(SB_PICK(kEvalFusedWide, F, E, T))                                \
+      if (threads > 512) SB_GO(SB_PICK(kEvalFusedWide, F, E, T, SB_COMMA 1024))                 \
+      if (threads > 256) SB_GO(SB_PICK(kEvalFusedWide, F, E, T, SB_COMMA 512))                  \
     }                                                                                           \
-    SB_GO(SB_PICK(kEvalFused, F, E, T))                                                         \
+    SB_GO(SB_PICK(kEvalFused, F, E, T, ))                                                       \
   }
 #define SB_TERMS(F, E)                                  \
   switch (terms) {                                      \
@@ -158,6 +161,7 @@ cudaError_t launchEvalFused(const DevSynthesis &d, int unit_begin, int unit_end,
   return cudaErrorInvalidValue;
 #undef SB_TERMS
 #undef SB_LAUNCH
+#undef SB_COMMA
 #undef SB_GO
 #undef SB_PICK
 }

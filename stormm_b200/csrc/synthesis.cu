@@ -1369,7 +1369,10 @@ void Synthesis::launchPlan(const UnitPlan &plan, int terms, bool force, bool ene
 //       against 145; 1,024: 71 against 75);
 //   512 when the launch evaluates every term and all its units are resident at two such blocks an
 //       SM, or its units average eight tiles and fit in one wave of 256-thread blocks (336 units of
-//       20-200 atoms: 70 us against 93; but 545 units of 24-96 atoms 64 against 48).
+//       20-200 atoms: 70 us against 93; but 545 units of 24-96 atoms 64 against 48);
+//   1,024 when a block per SM holds all the units and they average sixteen tiles (energies of 64
+//       molecules of 500-540 atoms: whole rescoring call 192 -> 177 us; 64 of 160-256 atoms,
+//       force and energy, 78 -> 74).
 // Sums are fixed-point, so the block size changes no result bit.
 int Synthesis::launchThreads(int units, int slots, long long tiles, int terms) const {
   if (opt.threads_per_block > 0 || !allow_wide) {
@@ -1377,6 +1380,9 @@ int Synthesis::launchThreads(int units, int slots, long long tiles, int terms) c
   }
   if (slots <= 128 && units > 5 * sm_count) {
     return 128;
+  }
+  if (terms == SB_TERM_ALL && units <= sm_count && tiles >= 16LL * units) {
+    return 1024;
   }
   if (terms == SB_TERM_ALL &&
       (units <= 2 * sm_count || (units < 4 * sm_count && tiles >= 8LL * units))) {

@@ -480,7 +480,7 @@ cudaError_t allowLargeSmem(K kern) {
 
 constexpr int kSlotBytes = 5 * 8 + 16 + 11 * 4;
 constexpr int kLateEntries = 128;   // per warp: pairs of a tile set aside before they are evaluated
-constexpr int kLateWarps = 16;      // warps of the largest block
+constexpr int kLateWarps = 32;      // warps of the largest block
 
 // Dynamic shared memory of one work unit's evaluation: max_slots atom slots, max_lj table entries
 __host__ __device__ inline size_t unitSmemBytes(int max_slots, int max_lj,

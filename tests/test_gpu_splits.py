@@ -67,3 +67,24 @@ def test_on_chip_minimizer_block_size_changes_no_bit():
         syn.close()
     for a, b in zip(*final):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.gpu
+def test_widest_blocks_change_no_bit():
+    """148 molecules of sixteen tiles and more take 1,024-thread blocks, 149 of them 512."""
+    import stormm_b200 as sb
+    from stormm_b200 import synthetic
+    mols = [synthetic.make_molecule(900 + k, n) for k, n in enumerate((193, 200, 224, 256))]
+    out = []
+    for count, threads in ((148, 1024), (149, 512)):
+        index = np.arange(count, dtype=np.int32) % len(mols)
+        syn = sb.Synthesis(mols, topology_index=index)
+        assert syn.launch_info()["threads"] == threads
+        syn.set_coordinates(np.concatenate([mols[t].coords for t in index]))
+        syn.initialize()
+        syn.evaluate()
+        out.append((syn.energies_fixed()[:148], syn.split(syn.forces())[:148]))
+        syn.close()
+    assert np.array_equal(out[0][0], out[1][0])
+    for a, b in zip(out[0][1], out[1][1]):
+        assert np.array_equal(a, b)
