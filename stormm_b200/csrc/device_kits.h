@@ -169,9 +169,20 @@ struct DevTiled {
   const int* atom_prefix;        // nmol + 1: first padded atom of each, counted over these only
   long long* psi_acc;            // per padded atom: psi at 2^kPsiBits
   long long* de_acc;             // per padded atom: dE/dR at 2^kDeijdaBits
-  float* radius;                 // per padded atom: effective GB radius
-  float* sde;                    // per padded atom: dE/dR after the chain-rule prefactor
+  // FP32 path: per 32 padded atoms the atom pair records that tile passes copy into shared memory
+  // (kBlockRecords float4), and a box (center; largest screened radius), (half extents; largest
+  // offset radius)
+  float4* records;
+  float4* boxes;
 };
+
+// Arrays of 16 records each within a block's kBlockRecords: hi and lo x / y, then z with the
+// payloads of passes 1 and 3 (s * rho, rho), z with those of pass 2 (charge, effective radius),
+// (1 / radius, Lennard-Jones code) of pass 2 and (unused, dE/dR) of pass 3
+enum BlockRecordArray : int {
+  kRecXY = 0, kRecXYLo, kRecZ1, kRecZ1Lo, kRecZ2, kRecZ2Lo, kRecG2, kRecG3, kRecArrays
+};
+constexpr int kBlockRecords = kRecArrays * kTile / 2;
 
 // Double-precision parameters of the FP64 mode (STORMM's double-precision kits beside the
 // single-precision ones), with the same layouts as their FP32 counterparts in DevSynthesis

@@ -1146,8 +1146,11 @@ void Synthesis::upload() {
   if (!h_tiled_systems.empty()) {
     arena.zero(&d_tiled_psi, natom_padded);
     arena.zero(&d_tiled_de, natom_padded);
-    arena.zero(&d_tiled_radius, natom_padded);
-    arena.zero(&d_tiled_sde, natom_padded);
+    if (!fp64) {
+      const size_t blocks = natom_padded / kTile;
+      arena.zero(&d_tiled_records, blocks * kBlockRecords);
+      arena.zero(&d_tiled_boxes, 2 * blocks);
+    }
   }
   if (fp64) {
     arena.put(&d64_charge, h64_charge);
@@ -1262,8 +1265,8 @@ void Synthesis::upload() {
   dev_tiled.atom_prefix = d_atom_prefix.p;
   dev_tiled.psi_acc = d_tiled_psi.p;
   dev_tiled.de_acc = d_tiled_de.p;
-  dev_tiled.radius = d_tiled_radius.p;
-  dev_tiled.sde = d_tiled_sde.p;
+  dev_tiled.records = d_tiled_records.p;
+  dev_tiled.boxes = d_tiled_boxes.p;
 
   DevSynthesis &d = dev;
   std::memset(&d, 0, sizeof(DevSynthesis));
@@ -1412,10 +1415,10 @@ void Synthesis::launchTiledRange(int mol_begin, int mol_end, int terms, bool for
   if (mol_end <= mol_begin) {
     return;
   }
-  const size_t np = natom_padded;
-  cudaCheck(cudaMemsetAsync(d_tiled_psi.p, 0, np * sizeof(long long), stream), "memset");
-  cudaCheck(cudaMemsetAsync(d_tiled_de.p, 0, np * sizeof(long long), stream), "memset");
   if (fp64) {
+    const size_t np = natom_padded;
+    cudaCheck(cudaMemsetAsync(d_tiled_psi.p, 0, np * sizeof(long long), stream), "memset");
+    cudaCheck(cudaMemsetAsync(d_tiled_de.p, 0, np * sizeof(long long), stream), "memset");
     DevPrecise p = dev64;
     p.clash_distance = clash.on() ? clash.distance64 : 0.0;
     p.clash_ratio = clash.on() ? clash.ratio64 : 0.0;

@@ -329,7 +329,7 @@ public:
   DeviceArray<int> d_sasa_cell, d_sasa_shape;
   DeviceArray<int> d_tiled_systems, d_tile_prefix, d_atom_prefix;
   DeviceArray<long long> d_tiled_psi, d_tiled_de;
-  DeviceArray<float> d_tiled_radius, d_tiled_sde;
+  DeviceArray<float4> d_tiled_records, d_tiled_boxes;
   DevTiled dev_tiled{};
   // FP64 mode (opt.precision == SB_PRECISION_DOUBLE): double parameters and per-atom GB state
   // (charges and 1-4 tables in double are built in both modes: FP32 valence uses them too)

@@ -239,13 +239,14 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __
 // (with each lane evaluating its own such pairs in turn, the busiest lane, with some eight, set the
 // cost and the gain was 1 %).
 // BRANCH: the polynomial behind a branch, for tiles where most steps have no pair within 4 sj.
+// FAR: every pair is known to lie beyond 4 sj and apart.
 constexpr float kSeriesLimit = 0.3f;
 
 struct Near2 {
   bool x, y;
 };
 
-template <bool DERIV, bool BRANCH>
+template <bool DERIV, bool BRANCH, bool FAR = false>
 __device__ __forceinline__ Near2 hctSeries2(float2 r, float2 invr, float2 rho, float2 sj,
                                             float2* integral, float2* deriv) {
   const float2 invr2 = mul2(invr, invr);
@@ -254,7 +255,7 @@ __device__ __forceinline__ Near2 hctSeries2(float2 r, float2 invr, float2 rho, f
   const bool near_x = t.x > 0.0625f;
   const bool near_y = t.y > 0.0625f;
   float2 ti = f2(0.0f), td = f2(0.0f);
-  if (!BRANCH || near_x || near_y) {
+  if (!FAR && (!BRANCH || near_x || near_y)) {
     ti = fma2(t, f2(1.4148261547e0f), f2(7.0001393557e-2f));
     ti = fma2(t, ti, f2(5.3365993500e-1f));
     ti = fma2(t, ti, f2(4.5760014653e-1f));
@@ -267,7 +268,7 @@ __device__ __forceinline__ Near2 hctSeries2(float2 r, float2 invr, float2 rho, f
       td = f2(near_x ? td.x : 0.0f, near_y ? td.y : 0.0f);
     }
   }
-  ti = fma2(t, ti, f2(kTaylorDD));
+  ti = FAR ? f2(kTaylorDD) : fma2(t, ti, f2(kTaylorDD));
   ti = fma2(t, ti, f2(kTaylorD));
   ti = fma2(t, ti, f2(kTaylorC));
   ti = fma2(t, ti, f2(kTaylorB));
@@ -275,12 +276,15 @@ __device__ __forceinline__ Near2 hctSeries2(float2 r, float2 invr, float2 rho, f
   const float2 scale = mul2(mul2(sj, t), invr2);
   *integral = mul2(scale, ti);
   if (DERIV) {
-    td = fma2(t, td, f2(kTaylorHH));
+    td = FAR ? f2(kTaylorHH) : fma2(t, td, f2(kTaylorHH));
     td = fma2(t, td, f2(kTaylorH));
     td = fma2(t, td, f2(kTaylorG));
     td = fma2(t, td, f2(kTaylorF));
     td = fma2(t, td, f2(kTaylorE));
     *deriv = mul2(mul2(scale, invr2), td);
+  }
+  if (FAR) {
+    return Near2{false, false};
   }
   // written so that a distance that is not a number is left to the closed forms, as before
   return Near2{!(r.x > touch.x && t.x <= kSeriesLimit), !(r.y > touch.y && t.y <= kSeriesLimit)};
@@ -1025,7 +1029,7 @@ __device__ __forceinline__ float2 diagonalWeights(const TileWalk &w, int lane, i
   return f2(1.0f, 1.0f);
 }
 
-// Run one tile: p.pair<false>(record, q, 1) for every step, or p.pair<true>(record, q, weights)
+// Run one tile: p.pair<false, .>(record, q, 1) for every step, or p.pair<true, .>(record, q, weights)
 // where pairs of weight 0 are to be left out, and p.rotate(source lane) after it.  Padding slots
 // hold parameters that make every contribution to a real atom exactly zero (no charge, zero
 // screened radius and dE/dR, masked Lennard-Jones, far-away coordinates), so partial tiles run the
@@ -1037,17 +1041,20 @@ __device__ __forceinline__ float2 diagonalWeights(const TileWalk &w, int lane, i
 template <class P>
 __device__ __forceinline__ void tileFlush(P &) {}
 
-template <class P>
+//
+// PLAIN (off-diagonal tiles of the tiled path): no pair of the tile is masked or closer than the
+// distances of tilePlain(), so the passes leave out what only near pairs need.
+template <bool PLAIN = false, class P>
 __device__ __forceinline__ void walkTile(P &p, const TileInfo &ti, const TileWalk &w, int lane) {
   const int jrec = slotRecord(ti.jbase);
   const int src = (lane & 16) | ((lane + 1) & 15);
   int q = w.q;
-  if (!w.diag) {
+  if (PLAIN || !w.diag) {
 #pragma unroll 1
     for (int k0 = 0; k0 < w.steps; k0 += 8) {
 #pragma unroll P::kUnroll
       for (int k = 0; k < 8; k++) {
-        p.template pair<false>(jrec + q, q, f2(1.0f));
+        p.template pair<false, PLAIN>(jrec + q, q, f2(1.0f));
         p.rotate(src);
         q = (q + 1) & 15;
       }
@@ -1057,7 +1064,7 @@ __device__ __forceinline__ void walkTile(P &p, const TileInfo &ti, const TileWal
   else {
 #pragma unroll 1
     for (int k = 0; k < w.steps; k++) {
-      p.template pair<true>(jrec + q, q, diagonalWeights(w, lane, k));
+      p.template pair<true, false>(jrec + q, q, diagonalWeights(w, lane, k));
       p.rotate(src);
       q = (q + 1) & 15;
       if (k == 4) {
@@ -1215,7 +1222,7 @@ struct RadiiPass {
     bit = 1u;
     out = tile_out;
   }
-  template <bool GUARD>
+  template <bool GUARD, bool PLAIN>
   __device__ __forceinline__ void pair(int rec, int q, float2 wt) {
     const float4 a = s.pa[rec], b = s.pb[rec], c = s.pc[rec], d = s.pd[rec];
     const Separation2 v = separate2<GUARD>(at, a, b, c, d, wt);
@@ -1223,11 +1230,11 @@ struct RadiiPass {
     const float2 r = mul2(v.r2, invr);
     const float2 rho_j = f2(d.z, d.w), s_j = f2(b.z, b.w);
     float2 hi, hj, di = f2(0.0f), dj = f2(0.0f);
-    const Near2 late_i = hctSeries2<STORE, BRANCH>(r, invr, rho_i, s_j, &hi, &di);
-    const Near2 late_j = hctSeries2<STORE, BRANCH>(r, invr, rho_j, s_i, &hj, &dj);
+    const Near2 late_i = hctSeries2<STORE, BRANCH, PLAIN>(r, invr, rho_i, s_j, &hi, &di);
+    const Near2 late_j = hctSeries2<STORE, BRANCH, PLAIN>(r, invr, rho_j, s_i, &hj, &dj);
     const bool late_x = late_i.x || late_j.x;
     const bool late_y = late_i.y || late_j.y;
-    if (NECK) {
+    if (NECK && !PLAIN) {
       if (!late_x && r.x < rho_i.x + rho_j.x + neck.reach) {
         const int nj = s.neck[jneck + q];
         float e, f;
@@ -1346,7 +1353,7 @@ struct PairPass {
     e_elec = e_vdw = e_gb = f2(0.0f);
     t_elec = t_vdw = t_gb = 0.0;
   }
-  template <bool GUARD>
+  template <bool GUARD, bool PLAIN>
   __device__ __forceinline__ void pair(int rec, int q, float2 wt) {
     const float4 a = s.pa[rec], b = s.pb[rec], c = s.pc[rec], d = s.pd[rec], g = s.pg[rec];
     const Separation2 v = separate2<GUARD>(at, a, b, c, d, wt);
@@ -1359,7 +1366,8 @@ struct PairPass {
     if (NB) {
       // excluded and padding pairs take the same path with zero parameters; nincl is -1 or 0
       const unsigned m = mask >> q;
-      float2 nincl = f2((m & 1u) ? 0.0f : -1.0f, (m & 0x10000u) ? 0.0f : -1.0f);
+      float2 nincl = PLAIN ? f2(-1.0f) :
+                             f2((m & 1u) ? 0.0f : -1.0f, (m & 0x10000u) ? 0.0f : -1.0f);
       if (GUARD) {
         nincl = mul2(nincl, wt);
       }
@@ -1369,17 +1377,24 @@ struct PairPass {
       // takes the exact r^2 = r2 + 2 (dx ex + dy ey + dz ez) + O(e^2), the e the separations'
       // recovered rounding errors (splitCoordinate): without it the Lennard-Jones energy of a
       // molecule with close contacts errs by up to 1.5e-6 of the root-sum-square of its pair
-      // terms.  r2 >= 256 on padding slots, never zero.
+      // terms.  r2 >= 256 on padding slots, never zero.  Beyond the distance of a plain tile the
+      // Lennard-Jones term is below 1e-5 of a contact's and takes the square of 1/r.
       float2 invr = f2(rsqrtf(r2.x), rsqrtf(r2.y));
       invr = mul2(invr, fma2(mul2(mul2(r2, f2(-0.5f)), invr), invr, f2(1.5f)));
-      const float2 ex = sub2(v.lx, sub2(v.dx, v.hx));
-      const float2 ey = sub2(v.ly, sub2(v.dy, v.hy));
-      const float2 ez = sub2(v.lz, sub2(v.dz, v.hz));
-      float2 m2r2c = fma2(v.dx, ex, fma2(v.dy, ey, mul2(v.dz, ez)));
-      m2r2c = mul2(m2r2c, f2(-2.0f));
-      float2 invr2 = f2(__fdividef(1.0f, r2.x), __fdividef(1.0f, r2.y));
-      const float2 step = fma2(m2r2c, invr2, fma2(mul2(r2, f2(-1.0f)), invr2, f2(1.0f)));
-      invr2 = fma2(invr2, step, invr2);
+      float2 invr2;
+      if (PLAIN) {
+        invr2 = mul2(invr, invr);
+      }
+      else {
+        const float2 ex = sub2(v.lx, sub2(v.dx, v.hx));
+        const float2 ey = sub2(v.ly, sub2(v.dy, v.hy));
+        const float2 ez = sub2(v.lz, sub2(v.dz, v.hz));
+        float2 m2r2c = fma2(v.dx, ex, fma2(v.dy, ey, mul2(v.dz, ez)));
+        m2r2c = mul2(m2r2c, f2(-2.0f));
+        invr2 = f2(__fdividef(1.0f, r2.x), __fdividef(1.0f, r2.y));
+        const float2 step = fma2(m2r2c, invr2, fma2(mul2(r2, f2(-1.0f)), invr2, f2(1.0f)));
+        invr2 = fma2(invr2, step, invr2);
+      }
       const float2 invr6 = mul2(mul2(invr2, invr2), invr2);
       const float2 ab1 = s.lj[code_i + (__float_as_int(g.z) >> 16)];
       const float2 ab2 = s.lj[code_i + (__float_as_int(g.w) >> 16)];
@@ -1505,7 +1520,7 @@ struct DerivPass {
     neck.both(z, a, r, invr, &dz);
     return da * de_a + dz * de_z;
   }
-  template <bool GUARD>
+  template <bool GUARD, bool PLAIN>
   __device__ __forceinline__ void pair(int rec, int q, float2 wt) {
     const float4 a = s.pa[rec], b = s.pb[rec], c = s.pc[rec], d = s.pd[rec], g = s.pg[rec];
     const Separation2 v = separate2<GUARD>(at, a, b, c, d, wt);
@@ -1513,12 +1528,12 @@ struct DerivPass {
     const float2 r = mul2(v.r2, invr);
     const float2 rho_j = f2(d.z, d.w), s_j = f2(b.z, b.w), de_j = f2(g.z, g.w);
     float2 unused, di, dj;
-    const Near2 late_i = hctSeries2<true, true>(r, invr, rho_i, s_j, &unused, &di);
-    const Near2 late_j = hctSeries2<true, true>(r, invr, rho_j, s_i, &unused, &dj);
+    const Near2 late_i = hctSeries2<true, true, PLAIN>(r, invr, rho_i, s_j, &unused, &di);
+    const Near2 late_j = hctSeries2<true, true, PLAIN>(r, invr, rho_j, s_i, &unused, &dj);
     const bool late_x = late_i.x || late_j.x;
     const bool late_y = late_i.y || late_j.y;
     float2 fmag = fma2(di, de_i, mul2(dj, de_j));
-    if (NECK) {
+    if (NECK && !PLAIN) {
       if (!late_x && r.x < rho_i.x + rho_j.x + neck.reach) {
         fmag.x += neckForce(ni, s.neck[jneck + q], r.x, invr.x, de_i.x, de_j.x);
       }
@@ -1585,7 +1600,7 @@ struct DerivStoredPass {
     fxj = fyj = fzj = f2(0.0f);
     in = tile_in;
   }
-  template <bool GUARD>
+  template <bool GUARD, bool PLAIN>
   __device__ __forceinline__ void pair(int rec, int, float2 wt) {
     const float4 hd = __ldcs(in);
     const float4 a = s.pa[rec], b = s.pb[rec], c = s.pc[rec], d = s.pd[rec], g = s.pg[rec];

@@ -60,3 +60,34 @@ def test_overlapping_pairs_beyond_the_list(route, natom, scale):
         err = np.abs(psi - ref["psi"])
         assert np.all(err <= 4.0e-6 * np.abs(ref["psi"]) + 1.0e-7), (force, err.max())
     syn.close()
+
+
+@pytest.mark.parametrize("grow", [1.0, 2.2])
+@pytest.mark.parametrize("gap", [5.0, 9.9, 10.04, 10.06, 13.0, 17.0])
+def test_plain_tiles_match_the_oracle(gap, grow):
+    """Two blocks of atoms `gap` apart, on both sides of the distance from which the tiled path
+    leaves out what only near pairs need (10 A, or four times the largest screened radius)."""
+    m = copy.deepcopy(synthetic.make_molecule(4200, 96))
+    rng = np.random.default_rng(7)
+    # three compact clusters in a row along x, one per block of 32 atoms
+    xyz = synthetic.make_molecule(4201, 32).coords
+    xyz = xyz - xyz.mean(axis=0)
+    width = np.ptp(xyz[:, 0])
+    m.coords = np.concatenate([xyz + [k * (width + gap), 0.0, 0.0] for k in range(3)])
+    m.coords = m.coords + rng.normal(0.0, 1.0e-3, size=m.coords.shape)
+    m.pb_radii = m.pb_radii * grow
+    m.excl12 = [set() for _ in range(96)]
+    m.excl13 = [set() for _ in range(96)]
+    m.excl14 = [set() for _ in range(96)]
+    if gap < 6.0:
+        m.excl12[3] = {70}
+        m.excl12[70] = {3}
+    terms = sb.TERM_NONBONDED | sb.TERM_GB
+    ref = oracle.from_molecule(m).evaluate(m.coords, terms=6)
+    syn = sb.Synthesis([m], tiled_above_atoms=32)
+    syn.set_coordinates(m.coords)
+    syn.initialize()
+    syn.evaluate(terms=terms)
+    check_energies(syn.energy_terms()[0], ref["energies"], oracle_magnitudes(m), (gap, grow))
+    assert rms_rel(syn.forces(), ref["forces"]) <= FORCE_TOL, (gap, grow)
+    syn.close()
