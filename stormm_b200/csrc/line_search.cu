@@ -4,9 +4,11 @@
 //   clear forces and energies, force + energy evaluation (kEvalFused)
 //   kLineStart    energy E0, gg / dgg / |f|^2, convergence, gamma, conjugate direction, its norm,
 //                 first trial move (conjugate_gradient.cui:8-140, line_movement.cui:88-126)
-//   clear energies, energy evaluation, kLineMove(1): E1, factor 1.04 or 0.8, second trial move
-//   clear energies, energy evaluation, kLineMove(2): E2, factor x1.03 or x0.85, third trial move
-//   clear energies, energy evaluation, kLineFinish: E3, cubic placement, next move length
+//   energy evaluation, kLineMove(1): E1, factor 1.04 or 0.8, second trial move
+//   energy evaluation, kLineMove(2): E2, factor x1.03 or x0.85, third trial move
+//   energy evaluation, kLineFinish: E3, cubic placement, next move length
+// kLineStart and kLineMove clear the energies they have read for the next evaluation (CLEAR; the
+// steps that a caller launches one by one leave them).
 // Each evaluation is the batched evaluation kernel at its best launch shape; the steps in between
 // are a warp per system with no block-wide barrier.  Per-system sums run over 32-atom chunks in
 // a fixed order, so a system's trajectory does not depend on the other systems of the batch.
@@ -29,11 +31,15 @@ __device__ __forceinline__ long long warpSumLong(long long v) {
   return v;
 }
 
-// Total potential energy of a system from its integer energy slots
+// Total potential energy of a system from its integer energy slots, which CLEAR then zeroes
+template <bool CLEAR = false>
 __device__ __forceinline__ double systemEnergy(const DevSynthesis &d, int sys, int lane) {
   long long v = 0;
   if (lane < kNrgStride) {
     v = static_cast<long long>(d.energies[static_cast<size_t>(sys) * kNrgStride + lane]);
+    if (CLEAR) {
+      d.energies[static_cast<size_t>(sys) * kNrgStride + lane] = 0ull;
+    }
   }
   return static_cast<double>(warpSumLong(v)) / static_cast<double>(d.nrg_scale);
 }
@@ -44,16 +50,24 @@ __device__ __forceinline__ int firstWarp() {
 
 __device__ __forceinline__ int warpStride() { return (gridDim.x * blockDim.x) >> 5; }
 
+// A system's line-search scalars, one per lane, fetched by one load; field() hands one to every lane
+struct LineScalars {
+  double mine;
+  __device__ __forceinline__ LineScalars(const double* line, int lane) :
+      mine(lane < kLineFields ? line[lane] : 0.0) {}
+  __device__ __forceinline__ double field(int f) const {
+    return __shfl_sync(0xffffffffu, mine, f);
+  }
+};
+
 // Move every atom of a system by step (fixed-point units per unit of direction); DBL: the FP64
 // mode's direction
 template <bool DBL>
-__device__ __forceinline__ void moveSystem(const DevSynthesis &d, const DevMinimizer &m, int sys,
+__device__ __forceinline__ void moveSystem(const DevMinimizer &m, int base, int natom,
                                            double step, int lane) {
   if (step == 0.0) {
     return;
   }
-  const int natom = d.atom_count[sys];
-  const int base = d.atom_start[sys];
   for (int a = lane; a < natom; a += 32) {
     const int gi = base + a;
     if (DBL) {
@@ -193,7 +207,7 @@ __device__ __forceinline__ void firstMove(const DevSynthesis &d, const DevMinimi
     line[kLineMv1] = 1.0;
   }
   __syncwarp();
-  moveSystem<DBL>(d, m, sys, inv_norm * s_move * gpos_scale, lane);
+  moveSystem<DBL>(m, d.atom_start[sys], d.atom_count[sys], inv_norm * s_move * gpos_scale, lane);
 }
 
 // Both at once, the graph minimizer's first line-search kernel of a cycle
@@ -202,7 +216,7 @@ __global__ void __launch_bounds__(kLineThreads)
 kLineStart(const DevSynthesis d, const DevMinimizer m, int first, int count) {
   const int lane = threadIdx.x & 31;
   for (int sys = first + firstWarp(); sys < first + count; sys += warpStride()) {
-    const double e0 = systemEnergy(d, sys, lane);
+    const double e0 = systemEnergy<true>(d, sys, lane);
     if (conjugateSystem<HIST, DBL>(d, m, sys, e0, lane)) {
       __syncwarp();
       const double inv_norm = m.line[static_cast<size_t>(sys) * kLineFields + kLineInvNorm];
@@ -237,33 +251,32 @@ kLineFirstMove(const DevSynthesis d, const DevMinimizer m, int first, int count)
 }
 
 // Second (move 1) or third (move 2) trial point
-template <bool DBL>
+template <bool DBL, bool CLEAR>
 __global__ void __launch_bounds__(kLineThreads)
 kLineMove(const DevSynthesis d, const DevMinimizer m, int first, int count, int move) {
   const int lane = threadIdx.x & 31;
   const double gpos_scale = 1.0 / d.inv_gpos_scale;
   for (int sys = first + firstWarp(); sys < first + count; sys += warpStride()) {
     double* line = m.line + static_cast<size_t>(sys) * kLineFields;
-    if (line[kLineAct] == 0.0) {
+    // every load that needs no result of another first: the kernel is a chain of latencies
+    const LineScalars scalars(line, lane);
+    const int base = d.atom_start[sys], natom = d.atom_count[sys];
+    const double e = systemEnergy<CLEAR>(d, sys, lane);
+    if (scalars.field(kLineAct) == 0.0) {
       continue;
     }
-    const double e = systemEnergy(d, sys, lane);
-    double mfac;
-    if (move == 1) {
-      mfac = (e < line[kLineE0]) ? 1.04 : 0.8;
-    }
-    else {
-      mfac = line[kLineMfac] * ((e < line[kLineE1]) ? 1.03 : 0.85);
-    }
-    const double mv_prev = (move == 1) ? line[kLineMv1] : line[kLineMv2];
-    const double step = line[kLineInvNorm] * mfac * line[kLineSMove] * gpos_scale;
-    __syncwarp();
+    const double before = scalars.field((move == 1) ? kLineE0 : kLineE1);
+    const double mfac = (move == 1) ? ((e < before) ? 1.04 : 0.8) :
+                                      scalars.field(kLineMfac) * ((e < before) ? 1.03 : 0.85);
+    const double mv_prev = scalars.field((move == 1) ? kLineMv1 : kLineMv2);
+    const double step = scalars.field(kLineInvNorm) * mfac * scalars.field(kLineSMove) *
+                        gpos_scale;
     if (lane == 0) {
       line[(move == 1) ? kLineE1 : kLineE2] = e;
       line[kLineMfac] = mfac;
       line[(move == 1) ? kLineMv2 : kLineMv3] = mv_prev + mfac;
     }
-    moveSystem<DBL>(d, m, sys, step, lane);
+    moveSystem<DBL>(m, base, natom, step, lane);
   }
 }
 
@@ -274,24 +287,27 @@ kLineFinish(const DevSynthesis d, const DevMinimizer m, int first, int count) {
   const int lane = threadIdx.x & 31;
   const double gpos_scale = 1.0 / d.inv_gpos_scale;
   for (int sys = first + firstWarp(); sys < first + count; sys += warpStride()) {
-    double* line = m.line + static_cast<size_t>(sys) * kLineFields;
-    if (line[kLineAct] == 0.0) {
+    const double* line = m.line + static_cast<size_t>(sys) * kLineFields;
+    const LineScalars scalars(line, lane);
+    const int base = d.atom_start[sys], natom = d.atom_count[sys];
+    const double e3 = systemEnergy(d, sys, lane);
+    if (scalars.field(kLineAct) == 0.0) {
       continue;
     }
-    const double e3 = systemEnergy(d, sys, lane);
-    const double ev[4] = {line[kLineE0], line[kLineE1], line[kLineE2], e3};
-    const double mv[4] = {0.0, line[kLineMv1], line[kLineMv2], line[kLineMv3]};
+    const double ev[4] = {scalars.field(kLineE0), scalars.field(kLineE1), scalars.field(kLineE2),
+                          e3};
+    const double mv[4] = {0.0, scalars.field(kLineMv1), scalars.field(kLineMv2),
+                          scalars.field(kLineMv3)};
     double new_base;
     const double mfac = finalPlacement(ev, mv, &new_base);
-    const double s_move = line[kLineSMove];
-    const double step = (fabs(mfac) > kVeryTiny) ?
-                        line[kLineInvNorm] * mfac * s_move * gpos_scale : 0.0;
-    __syncwarp();
+    const double s_move = scalars.field(kLineSMove);
+    const double inv_norm = scalars.field(kLineInvNorm);
+    const double step = (fabs(mfac) > kVeryTiny) ? inv_norm * mfac * s_move * gpos_scale : 0.0;
     if (lane == 0) {
       m.l_move[sys] = s_move * new_base;
       m.cycle[sys] += 1;
     }
-    moveSystem<DBL>(d, m, sys, step, lane);
+    moveSystem<DBL>(m, base, natom, step, lane);
   }
 }
 
@@ -317,9 +333,11 @@ int lineGrid(int count) {
 }  // namespace
 
 // step: 0 start (conjugate gradient and first move), 1 and 2 trial moves, 3 finish, 4 history
-// of the final energies, 5 the conjugate-gradient step alone, 6 the first move alone
+// of the final energies, 5 the conjugate-gradient step alone, 6 the first move alone.  clear: steps
+// 1 and 2 as part of the graph minimizer's cycle, which clear the energies they read (step 0 always
+// does)
 cudaError_t launchLineStep(const DevSynthesis &d, const DevMinimizer &m, int first, int count,
-                           int step, cudaStream_t stream) {
+                           int step, bool clear, cudaStream_t stream) {
   if (count <= 0) {
     return cudaSuccess;
   }
@@ -345,10 +363,12 @@ cudaError_t launchLineStep(const DevSynthesis &d, const DevMinimizer &m, int fir
     case 1:
     case 2:
       if (dbl) {
-        kLineMove<true><<<grid, kLineThreads, 0, stream>>>(d, m, first, count, step);
+        auto kern = clear ? kLineMove<true, true> : kLineMove<true, false>;
+        kern<<<grid, kLineThreads, 0, stream>>>(d, m, first, count, step);
       }
       else {
-        kLineMove<false><<<grid, kLineThreads, 0, stream>>>(d, m, first, count, step);
+        auto kern = clear ? kLineMove<false, true> : kLineMove<false, false>;
+        kern<<<grid, kLineThreads, 0, stream>>>(d, m, first, count, step);
       }
       break;
     case 3:

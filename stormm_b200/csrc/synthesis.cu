@@ -34,7 +34,7 @@ cudaError_t launchMinimize(const DevSynthesis &d, const DevMinimizer &m, int uni
                            int unit_end, int max_lj, int cycles, bool final_energy, int threads,
                            int sm_count, cudaStream_t stream);
 cudaError_t launchLineStep(const DevSynthesis &d, const DevMinimizer &m, int first, int count,
-                           int step, cudaStream_t stream);
+                           int step, bool clear, cudaStream_t stream);
 cudaError_t launchTiled(const DevSynthesis &d, const DevTiled &t, const int* h_tile_prefix,
                         const int* h_atom_prefix, int mol_begin, int mol_end, int terms,
                         bool force, bool energy, bool workspace, int sm_count,
@@ -1852,17 +1852,14 @@ void Synthesis::evaluateFor(int first, int count, bool single, bool force, cudaS
 }
 
 // One graph-mode cycle: evaluations by the batched evaluation kernel, line-search steps by a warp
-// per system (line_search.cu)
+// per system (line_search.cu); each step but the last clears the energies for the next evaluation
 void Synthesis::graphCycle(int first, int count, bool single, cudaStream_t stream) {
-  const size_t nrg_bytes = d_energies.n * sizeof(unsigned long long);
   const Clash clash = minimizerClash();
   initialize(SB_INIT_FORCES | SB_INIT_ENERGIES, stream);
-  evaluateFor(first, count, single, true, stream, clash);
-  cudaCheck(launchLineStep(dev, dev_min, first, count, 0, stream), "line search launch");
-  for (int step = 1; step <= 3; step++) {
-    cudaCheck(cudaMemsetAsync(d_energies.p, 0, nrg_bytes, stream), "memset");
-    evaluateFor(first, count, single, false, stream, clash);
-    cudaCheck(launchLineStep(dev, dev_min, first, count, step, stream), "line search launch");
+  for (int step = 0; step <= 3; step++) {
+    evaluateFor(first, count, single, step == 0, stream, clash);
+    cudaCheck(launchLineStep(dev, dev_min, first, count, step, true, stream),
+              "line search launch");
   }
 }
 
@@ -1871,7 +1868,7 @@ void Synthesis::graphFinalEnergy(int first, int count, bool single, cudaStream_t
   cudaCheck(cudaMemsetAsync(d_energies.p, 0, d_energies.n * sizeof(unsigned long long), stream),
             "memset");
   evaluateFor(first, count, single, false, stream);
-  cudaCheck(launchLineStep(dev, dev_min, first, count, 4, stream), "line search launch");
+  cudaCheck(launchLineStep(dev, dev_min, first, count, 4, false, stream), "line search launch");
 }
 
 void Synthesis::checkMinimizeSmem(int slots, int lj) const {
@@ -1913,7 +1910,7 @@ void Synthesis::conjugateGradient(cudaStream_t stream) {
   if (!min_ready) {
     throw Error(SB_ERR_ARGUMENT, "no minimization has begun on this synthesis");
   }
-  cudaCheck(launchLineStep(dev, dev_min, 0, nsys, 5, stream), "conjugate gradient launch");
+  cudaCheck(launchLineStep(dev, dev_min, 0, nsys, 5, false, stream), "conjugate gradient launch");
 }
 
 void Synthesis::lineAdvance(int move, cudaStream_t stream) {
@@ -1923,7 +1920,7 @@ void Synthesis::lineAdvance(int move, cudaStream_t stream) {
   if (move < 0 || move > 3) {
     throw Error(SB_ERR_ARGUMENT, "line move number must be 0, 1, 2 or 3");
   }
-  cudaCheck(launchLineStep(dev, dev_min, 0, nsys, (move == 0) ? 6 : move, stream),
+  cudaCheck(launchLineStep(dev, dev_min, 0, nsys, (move == 0) ? 6 : move, false, stream),
             "line advance launch");
 }
 
