@@ -22,8 +22,9 @@
 
 namespace sb {
 
-// Dynamic shared memory needed for a work unit of max_slots atom slots and max_lj table entries
-size_t fusedSmemBytes(int max_slots, int max_lj) { return unitSmemBytes(max_slots, max_lj); }
+// Most dynamic shared memory any block takes for a work unit of max_slots atom slots and max_lj
+// table entries
+size_t fusedSmemBytes(int max_slots, int max_lj) { return unitSmemBytes(max_slots, max_lj, 1024); }
 
 // ------------------------------------------------------------------------------------------------
 // The fused kernel: stage, evaluate, commit, one work unit at a time
@@ -105,7 +106,6 @@ kEvalFusedWide(const DevSynthesis d, int unit_begin, int unit_end, int max_lj) {
 cudaError_t launchEvalFused(const DevSynthesis &d, int unit_begin, int unit_end, int max_lj,
                             int terms, bool force, bool energy, int blocks, int threads,
                             cudaStream_t stream, bool clash) {
-  const size_t smem = fusedSmemBytes(d.max_unit_slots, max_lj);
   // softened cores change only Coulomb, Lennard-Jones and 1-4 terms, the neck term only GB
   clash = clash && (terms & 3) != 0;
   const bool neck = d.neck_size > 0 && (terms & 4) != 0;
@@ -116,6 +116,7 @@ cudaError_t launchEvalFused(const DevSynthesis &d, int unit_begin, int unit_end,
   if (threads != 512 && threads != 1024 && (threads < 64 || threads > 256 || threads % 32 != 0)) {
     return cudaErrorInvalidValue;
   }
+  const size_t smem = unitSmemBytes(d.max_unit_slots, max_lj, threads);
 #define SB_PICK(K, F, E, T, ...)                                                                \
     (neck ? (clash ? K<F, E, T, ((T) & 3) != 0, ((T) & 4) != 0 __VA_ARGS__> :                   \
                      K<F, E, T, false, ((T) & 4) != 0 __VA_ARGS__>) :                           \

@@ -325,10 +325,10 @@ __device__ void minimizationCycle(const DevSynthesis &d, const DevMinimizer &m,
 // Every cycle of one work unit, then its final energies (undamped) and state
 template <bool CLASH, bool NECK, class Team>
 __device__ void minimizeUnit(const DevSynthesis &d, const DevMinimizer &m, const UnitSmem &s,
-                             const MinSmem &ms, int u, int max_lj, int max_sys, int cycles,
-                             int final_energy, const Team &team) {
+                             const MinSmem &ms, int u, int max_lj, int cycles, int final_energy,
+                             const Team &team) {
   UnitShape us;
-  if (!stageUnitTables(d, s, u, max_lj, &us, team, max_sys)) {
+  if (!stageUnitTables(d, s, u, max_lj, &us, team)) {
     return;
   }
   for (int slot = team.rank(); slot < us.nslots; slot += team.size()) {
@@ -393,14 +393,13 @@ kMinimize(const DevSynthesis d, const DevMinimizer m, int unit_begin, int unit_e
           int cycles, int final_energy) {
   extern __shared__ __align__(16) char smem_raw[];
   const UnitSmem s = carveSmem(smem_raw, d.max_unit_slots, max_lj);
-  const MinSmem ms = carveMinSmem(smem_raw + unitSmemBytes(d.max_unit_slots, max_lj),
-                                  d.max_unit_slots, kMaxUnitSystems);
+  const MinSmem ms = carveMinSmem(smem_raw + unitSmemBytes(d.max_unit_slots, max_lj, blockDim.x),
+                                  d.max_unit_slots, unitSystems(d.max_unit_slots));
   __shared__ int next_unit;
   const BlockTeam team;
   int u = unit_begin + blockIdx.x;
   while (u < unit_end) {
-    minimizeUnit<CLASH, NECK>(d, m, s, ms, u, max_lj, kMaxUnitSystems, cycles,
-                                    final_energy, team);
+    minimizeUnit<CLASH, NECK>(d, m, s, ms, u, max_lj, cycles, final_energy, team);
     if (threadIdx.x == 0) {
       next_unit = unit_begin + static_cast<int>(gridDim.x) + atomicAdd(m.queue, 1);
     }
@@ -434,8 +433,8 @@ __global__ void kMinimizerReset(DevMinimizer m, int nsys, int natom_padded, doub
 
 }  // namespace
 
-size_t minimizeSmemBytes(int max_slots, int max_lj) {
-  return unitSmemBytes(max_slots, max_lj) + minSmemBytes(max_slots, kMaxUnitSystems);
+size_t minimizeSmemBytes(int max_slots, int max_lj, int threads) {
+  return unitSmemBytes(max_slots, max_lj, threads) + minSmemBytes(max_slots, unitSystems(max_slots));
 }
 
 
@@ -456,7 +455,7 @@ cudaError_t launchMinimize(const DevSynthesis &d, const DevMinimizer &m, int uni
   if (unit_end <= unit_begin) {
     return cudaSuccess;
   }
-  const size_t smem = minimizeSmemBytes(d.max_unit_slots, max_lj);
+  const size_t smem = minimizeSmemBytes(d.max_unit_slots, max_lj, threads);
   const bool clash = m.clash_cycles > 0 && (m.clash_distance > 0.0f || m.clash_ratio > 0.0f);
   const bool neck = d.neck_size > 0;
   auto pick = [&](auto threads_c) {

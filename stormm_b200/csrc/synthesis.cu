@@ -27,7 +27,7 @@ size_t fusedSmemBytes(int max_slots, int max_lj);
 cudaError_t launchEvalFused(const DevSynthesis &d, int unit_begin, int unit_end, int max_lj,
                             int terms, bool force, bool energy, int blocks, int threads,
                             cudaStream_t stream, bool clash);
-size_t minimizeSmemBytes(int max_slots, int max_lj);
+size_t minimizeSmemBytes(int max_slots, int max_lj, int threads);
 cudaError_t launchMinimizerReset(const DevMinimizer &m, const DevSynthesis &d, double dx0,
                                  cudaStream_t stream);
 cudaError_t launchMinimize(const DevSynthesis &d, const DevMinimizer &m, int unit_begin,
@@ -1872,7 +1872,7 @@ void Synthesis::graphFinalEnergy(int first, int count, bool single, cudaStream_t
 }
 
 void Synthesis::checkMinimizeSmem(int slots, int lj) const {
-  if (static_cast<int>(minimizeSmemBytes(slots, lj)) > max_smem_optin) {
+  if (static_cast<int>(minimizeSmemBytes(slots, lj, 512)) > max_smem_optin) {
     throw Error(SB_ERR_UNSUPPORTED, "a molecule is too large for on-chip minimization");
   }
 }

@@ -484,11 +484,17 @@ cudaError_t allowLargeSmem(K kern) {
 
 constexpr int kSlotBytes = 5 * 8 + 16 + 11 * 4;
 constexpr int kLateEntries = 128;   // per warp: pairs of a tile set aside before they are evaluated
-constexpr int kLateWarps = 32;      // warps of the largest block
 
-// Dynamic shared memory of one work unit's evaluation: max_slots atom slots, max_lj table entries
-__host__ __device__ inline size_t unitSmemBytes(int max_slots, int max_lj,
-                                                int max_sys = kMaxUnitSystems) {
+// Most molecules a work unit of max_slots atom slots can hold (each takes at least a tile's edge)
+__host__ __device__ inline int unitSystems(int max_slots) {
+  const int n = max_slots / kTile;
+  return n < kMaxUnitSystems ? n : kMaxUnitSystems;
+}
+
+// Dynamic shared memory of one work unit's evaluation by a block of `threads`: max_slots atom slots,
+// max_lj table entries
+__host__ __device__ inline size_t unitSmemBytes(int max_slots, int max_lj, int threads) {
+  const int max_sys = unitSystems(max_slots);
   size_t b = static_cast<size_t>(kSlotBytes) * max_slots;
   b = alignUp(b, 16);
   b += sizeof(float2) * max_lj;
@@ -496,12 +502,12 @@ __host__ __device__ inline size_t unitSmemBytes(int max_slots, int max_lj,
   b += sizeof(unsigned long long) * max_sys * kNrgStride;
   b += sizeof(float2) * max_sys;
   b += sizeof(int) * kUnitMetaFields * (max_sys + 1);
-  b += sizeof(unsigned short) * kLateEntries * kLateWarps;
+  b += sizeof(unsigned short) * kLateEntries * (threads / 32);
   return alignUp(b, 16);
 }
 
-__device__ UnitSmem carveSmem(char* base, int max_slots, int max_lj,
-                              int max_sys = kMaxUnitSystems) {
+__device__ UnitSmem carveSmem(char* base, int max_slots, int max_lj) {
+  const int max_sys = unitSystems(max_slots);
   UnitSmem s;
   size_t off = 0;
   const size_t records = sizeof(float4) * (max_slots / 2);
@@ -1825,7 +1831,8 @@ struct UnitShape {
 // caller then skips the unit.  Ends with a barrier.
 template <class Team>
 __device__ bool stageUnitTables(const DevSynthesis &d, const UnitSmem &s, int u, int max_lj,
-                                UnitShape* shape, const Team &team, int max_sys = kMaxUnitSystems) {
+                                UnitShape* shape, const Team &team) {
+  const int max_sys = s.metaStride - 1;
   const int4 desc = d.unit_desc[u];
   const int nsys_u = desc.y;
   shape->nsys = nsys_u;
