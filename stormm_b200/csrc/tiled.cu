@@ -13,6 +13,7 @@
 // molecule.
 #include <cuda_runtime.h>
 
+#include "launch.cuh"
 #include "unit_eval.cuh"
 #include "tile_tasks.cuh"
 
@@ -100,6 +101,7 @@ struct GlobalValence {
 template <bool FORCE, bool ENERGY, bool CLASH>
 __global__ void __launch_bounds__(256)
 kTiledValence(const DevSynthesis d, const DevTiled t, int mol_begin) {
+  gridWait();
   valenceTerms<FORCE, ENERGY, GlobalValence, CLASH>(
       d, GlobalValence(d, t.systems[mol_begin + blockIdx.x]));
 }
@@ -117,6 +119,7 @@ __device__ __forceinline__ float &blockValue(const DevTiled &t, int gi, int arr,
 // 32 chains of 2,000-5,000 atoms, force + energy with copies, 1,600 -> 1,318 us.
 __global__ void __launch_bounds__(256)
 kTiledPrepare(const DevSynthesis d, const DevTiled t, int atom_begin, int atom_end) {
+  gridWait();
   const int lane = threadIdx.x & 31;
   for (int q = atom_begin + blockIdx.x * blockDim.x + threadIdx.x; q < atom_end;
        q += gridDim.x * blockDim.x) {
@@ -255,6 +258,7 @@ __device__ __forceinline__ void addGlobal(long long* acc, float v) {
 template <bool NECK>
 __global__ void __launch_bounds__(256, 4)
 kTiledRadii(const DevSynthesis d, const DevTiled t, int tile_begin, int tile_end) {
+  gridWait();
   __shared__ TileStage stage;
   const int lane = threadIdx.x & 31;
   const float ps = static_cast<float>(1 << kPsiBits);
@@ -297,6 +301,7 @@ kTiledRadii(const DevSynthesis d, const DevTiled t, int tile_begin, int tile_end
 template <bool FORCE, bool ENERGY, bool NB, bool GB, bool CLASH>
 __global__ void __launch_bounds__(256, 3)
 kTiledPair(const DevSynthesis d, const DevTiled t, int tile_begin, int tile_end) {
+  gridWait();
   __shared__ TileStage stage;
   const int lane = threadIdx.x & 31;
   const float fs = d.frc_scale;
@@ -402,6 +407,7 @@ kTiledPair(const DevSynthesis d, const DevTiled t, int tile_begin, int tile_end)
 template <bool NECK>
 __global__ void __launch_bounds__(256, 4)
 kTiledDeriv(const DevSynthesis d, const DevTiled t, int tile_begin, int tile_end) {
+  gridWait();
   __shared__ TileStage stage;
   const int lane = threadIdx.x & 31;
   const float fs = d.frc_scale;
@@ -451,6 +457,7 @@ kTiledDeriv(const DevSynthesis d, const DevTiled t, int tile_begin, int tile_end
 template <bool FORCE, bool ENERGY, bool WS>
 __global__ void __launch_bounds__(256)
 kTiledAtoms(const DevSynthesis d, const DevTiled t, int atom_begin, int atom_end) {
+  gridWait();
   const float inv_ps = 1.0f / static_cast<float>(1 << kPsiBits);
   const float ds = static_cast<float>(1 << kDeijdaBits);
   for (int q = atom_begin + blockIdx.x * blockDim.x + threadIdx.x; q < atom_end;
@@ -488,6 +495,7 @@ kTiledAtoms(const DevSynthesis d, const DevTiled t, int atom_begin, int atom_end
 template <bool WS>
 __global__ void __launch_bounds__(256)
 kTiledChain(const DevSynthesis d, const DevTiled t, int atom_begin, int atom_end) {
+  gridWait();
   const float inv_ds = 1.0f / static_cast<float>(1 << kDeijdaBits);
   const float inv_ps = 1.0f / static_cast<float>(1 << kPsiBits);
   for (int q = atom_begin + blockIdx.x * blockDim.x + threadIdx.x; q < atom_end;
@@ -535,22 +543,22 @@ cudaError_t launchTiled(const DevSynthesis &d, const DevTiled &t, const int* h_t
     vrows = vrows < 4 ? 4 : (vrows > 32 ? 32 : vrows);
     const dim3 vgrid(nmol, vrows);
 #define SB_VALE(C)                                                                             \
-    if (force && energy) kTiledValence<true, true, C><<<vgrid, 256, 0, stream>>>(d, t, mol_begin); \
-    else if (force) kTiledValence<true, false, C><<<vgrid, 256, 0, stream>>>(d, t, mol_begin);   \
-    else kTiledValence<false, true, C><<<vgrid, 256, 0, stream>>>(d, t, mol_begin);
+    if (force && energy) launchAfter(kTiledValence<true, true, C>, vgrid, 256, 0, stream, d, t, mol_begin); \
+    else if (force) launchAfter(kTiledValence<true, false, C>, vgrid, 256, 0, stream, d, t, mol_begin);   \
+    else launchAfter(kTiledValence<false, true, C>, vgrid, 256, 0, stream, d, t, mol_begin);
     if (clash) { SB_VALE(true) }
     else { SB_VALE(false) }
 #undef SB_VALE
   }
   if (nb || gb) {
-    kTiledPrepare<<<agrid, 256, 0, stream>>>(d, t, ab, ae);
+    launchAfter(kTiledPrepare, agrid, 256, 0, stream, d, t, ab, ae);
   }
   if (gb) {
-    if (d.neck_size > 0) kTiledRadii<true><<<tgrid, 256, 0, stream>>>(d, t, tb, te);
-    else kTiledRadii<false><<<tgrid, 256, 0, stream>>>(d, t, tb, te);
+    if (d.neck_size > 0) launchAfter(kTiledRadii<true>, tgrid, 256, 0, stream, d, t, tb, te);
+    else launchAfter(kTiledRadii<false>, tgrid, 256, 0, stream, d, t, tb, te);
 #define SB_ATOMS(F, E) \
-    if (workspace) kTiledAtoms<F, E, true><<<agrid, 256, 0, stream>>>(d, t, ab, ae); \
-    else kTiledAtoms<F, E, false><<<agrid, 256, 0, stream>>>(d, t, ab, ae);
+    if (workspace) launchAfter(kTiledAtoms<F, E, true>, agrid, 256, 0, stream, d, t, ab, ae); \
+    else launchAfter(kTiledAtoms<F, E, false>, agrid, 256, 0, stream, d, t, ab, ae);
     if (force && energy) { SB_ATOMS(true, true) }
     else if (force) { SB_ATOMS(true, false) }
     else { SB_ATOMS(false, true) }
@@ -558,9 +566,9 @@ cudaError_t launchTiled(const DevSynthesis &d, const DevTiled &t, const int* h_t
   }
   if (nb || gb) {
 #define SB_PAIR(F, E, C)                                                                      \
-    if (nb && gb) kTiledPair<F, E, true, true, C><<<tgrid, 256, 0, stream>>>(d, t, tb, te);    \
-    else if (nb) kTiledPair<F, E, true, false, C><<<tgrid, 256, 0, stream>>>(d, t, tb, te);   \
-    else kTiledPair<F, E, false, true, false><<<tgrid, 256, 0, stream>>>(d, t, tb, te);
+    if (nb && gb) launchAfter(kTiledPair<F, E, true, true, C>, tgrid, 256, 0, stream, d, t, tb, te);    \
+    else if (nb) launchAfter(kTiledPair<F, E, true, false, C>, tgrid, 256, 0, stream, d, t, tb, te);   \
+    else launchAfter(kTiledPair<F, E, false, true, false>, tgrid, 256, 0, stream, d, t, tb, te);
     if (clash) {
       if (force && energy) { SB_PAIR(true, true, true) }
       else if (force) { SB_PAIR(true, false, true) }
@@ -574,10 +582,10 @@ cudaError_t launchTiled(const DevSynthesis &d, const DevTiled &t, const int* h_t
 #undef SB_PAIR
   }
   if (gb && force) {
-    if (workspace) kTiledChain<true><<<agrid, 256, 0, stream>>>(d, t, ab, ae);
-    else kTiledChain<false><<<agrid, 256, 0, stream>>>(d, t, ab, ae);
-    if (d.neck_size > 0) kTiledDeriv<true><<<tgrid, 256, 0, stream>>>(d, t, tb, te);
-    else kTiledDeriv<false><<<tgrid, 256, 0, stream>>>(d, t, tb, te);
+    if (workspace) launchAfter(kTiledChain<true>, agrid, 256, 0, stream, d, t, ab, ae);
+    else launchAfter(kTiledChain<false>, agrid, 256, 0, stream, d, t, ab, ae);
+    if (d.neck_size > 0) launchAfter(kTiledDeriv<true>, tgrid, 256, 0, stream, d, t, tb, te);
+    else launchAfter(kTiledDeriv<false>, tgrid, 256, 0, stream, d, t, tb, te);
   }
   return cudaGetLastError();
 }

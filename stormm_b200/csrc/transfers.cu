@@ -9,6 +9,7 @@
 
 #include "device_kits.h"
 #include "fixed_point.cuh"
+#include "launch.cuh"
 
 namespace sb {
 
@@ -18,6 +19,7 @@ namespace {
 __global__ void kImportCoordinates(const double* __restrict__ xyz, const int* __restrict__ map,
                                    int natom, double scale, long long* xcrd, long long* ycrd,
                                    long long* zcrd, int* xo, int* yo, int* zo, int* status) {
+  gridWait();
   for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < natom; a += gridDim.x * blockDim.x) {
     const int gi = map[a];
     const double x = xyz[3 * a] * scale;
@@ -43,6 +45,7 @@ __global__ void kExportCoordinates(const long long* __restrict__ xcrd,
                                    const long long* __restrict__ zcrd,
                                    const int* __restrict__ map, int natom, double inv_scale,
                                    double* xyz) {
+  gridWait();
   for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < natom; a += gridDim.x * blockDim.x) {
     const int gi = map[a];
     xyz[3 * a] = static_cast<double>(xcrd[gi]) * inv_scale;
@@ -56,6 +59,7 @@ __global__ void kExportForces(const long long* __restrict__ xf, const long long*
                               const int* __restrict__ yo, const int* __restrict__ zo,
                               const int* __restrict__ map, int natom, double inv_scale,
                               double* xyz) {
+  gridWait();
   for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < natom; a += gridDim.x * blockDim.x) {
     const int gi = map[a];
     xyz[3 * a] = int95ToDouble(xf[gi], xo[gi]) * inv_scale;
@@ -66,6 +70,7 @@ __global__ void kExportForces(const long long* __restrict__ xf, const long long*
 
 __global__ void kExportEnergies(const unsigned long long* __restrict__ nrg, int n,
                                 double inv_scale, double* out) {
+  gridWait();
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
     out[e] = static_cast<double>(static_cast<long long>(nrg[e])) * inv_scale;
   }
@@ -73,6 +78,7 @@ __global__ void kExportEnergies(const unsigned long long* __restrict__ nrg, int 
 
 // Zero several arrays in one launch: each block walks every array in 16-byte words
 __global__ void kClear(ClearList list) {
+  gridWait();
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
   for (int a = 0; a < list.count; a++) {
@@ -96,7 +102,7 @@ cudaError_t launchImportCoordinates(const double* d_xyz, const int* d_map, int n
                                     double scale, long long* xcrd, long long* ycrd,
                                     long long* zcrd, int* xo, int* yo, int* zo, int* status,
                                     cudaStream_t stream) {
-  kImportCoordinates<<<gridFor(natom), 256, 0, stream>>>(d_xyz, d_map, natom, scale, xcrd, ycrd,
+  launchAfter(kImportCoordinates, gridFor(natom), 256, 0, stream, d_xyz, d_map, natom, scale, xcrd, ycrd,
                                                          zcrd, xo, yo, zo, status);
   return cudaGetLastError();
 }
@@ -104,7 +110,7 @@ cudaError_t launchImportCoordinates(const double* d_xyz, const int* d_map, int n
 cudaError_t launchExportCoordinates(const long long* xcrd, const long long* ycrd,
                                     const long long* zcrd, const int* d_map, int natom,
                                     double inv_scale, double* d_xyz, cudaStream_t stream) {
-  kExportCoordinates<<<gridFor(natom), 256, 0, stream>>>(xcrd, ycrd, zcrd, d_map, natom,
+  launchAfter(kExportCoordinates, gridFor(natom), 256, 0, stream, xcrd, ycrd, zcrd, d_map, natom,
                                                          inv_scale, d_xyz);
   return cudaGetLastError();
 }
@@ -112,7 +118,7 @@ cudaError_t launchExportCoordinates(const long long* xcrd, const long long* ycrd
 cudaError_t launchExportForces(const long long* xf, const long long* yf, const long long* zf,
                                const int* xo, const int* yo, const int* zo, const int* d_map,
                                int natom, double inv_scale, double* d_xyz, cudaStream_t stream) {
-  kExportForces<<<gridFor(natom), 256, 0, stream>>>(xf, yf, zf, xo, yo, zo, d_map, natom,
+  launchAfter(kExportForces, gridFor(natom), 256, 0, stream, xf, yf, zf, xo, yo, zo, d_map, natom,
                                                     inv_scale, d_xyz);
   return cudaGetLastError();
 }
@@ -127,13 +133,13 @@ cudaError_t launchClear(const ClearList &list, int sm_count, cudaStream_t stream
   size_t blocks = (most + 255) / 256;
   const size_t cap = static_cast<size_t>(sm_count > 0 ? sm_count : 148) * 8;
   blocks = (blocks > cap) ? cap : blocks;
-  kClear<<<static_cast<int>(blocks), 256, 0, stream>>>(list);
+  launchAfter(kClear, static_cast<int>(blocks), 256, 0, stream, list);
   return cudaGetLastError();
 }
 
 cudaError_t launchExportEnergies(const unsigned long long* nrg, int n, double inv_scale,
                                  double* d_out, cudaStream_t stream) {
-  kExportEnergies<<<gridFor(n), 256, 0, stream>>>(nrg, n, inv_scale, d_out);
+  launchAfter(kExportEnergies, gridFor(n), 256, 0, stream, nrg, n, inv_scale, d_out);
   return cudaGetLastError();
 }
 
