@@ -6,12 +6,12 @@
 // one before it before it ends, the order of the whole chain is kept.  After a kernel or a copy
 // that gives no such signal the launch is an ordinary one.
 //
-// Taken by the tiled path, whose evaluation of one chain is eight short kernels in a row, and the
-// copies' conversion kernels (one 2,500-atom chain with copies 116 -> 97 us; 1,024 molecules, clearing and
-// export kernels alone, 389 -> 379).  Not by the fused
-// evaluation, whose large units come first and are then placed on the SMs that happen to be free
-// (1,024 molecules 389 -> 436 us), the FP64 passes (128 molecules 206 -> 216) or the minimizer's cycle
-// graph (one molecule, 60 cycles 4.38 -> 4.59 ms).
+// Taken by the tiled path, whose evaluation of one chain is eight short kernels in a row, and by the
+// clearing and conversion kernels (one 2,500-atom chain with copies 116 -> 98 us; 1,024 molecules,
+// through the latter alone, 389 -> 380).  Not by the fused evaluation, whose large units come first
+// and are then placed on the SMs that happen to be free (1,024 molecules 389 -> 436 us), the FP64
+// passes (128 molecules 206 -> 216) or the minimizer's cycle graph (one molecule, 60 cycles 4.38 ->
+// 4.59 ms).
 #ifndef STORMM_B200_LAUNCH_CUH
 #define STORMM_B200_LAUNCH_CUH
 

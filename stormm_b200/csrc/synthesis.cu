@@ -1062,8 +1062,8 @@ void Synthesis::buildUnits() {
   // Minimization keeps whole molecules on chip for hundreds of cycles.  A batch of at most one
   // molecule per SM gives each its own block, in one launch and with 512 threads (launchMinPlan):
   // such a launch lasts as long as its largest molecule.  128 molecules of 12-512 atoms, 60 cycles:
-  // one launch after another with 256 threads 16.8 ms, this way 8.2 ms.  Larger batches share units of up to 128 slots, which balance the persistent grid
-  // (sb_autotune can choose another packing).
+  // one launch after another with 256 threads 16.8 ms, this way 8.3 ms.  Larger batches share units
+  // of up to 128 slots, which balance the persistent grid (sb_autotune can choose another packing).
   min_plan = (nfused <= sm_count) ? makePlan(std::max(widest, kTile), 1, true) :
                                     makePlan(128, 16, true);
   // one unit per system, in system order, for the per-system launches
