@@ -286,7 +286,8 @@ __device__ __forceinline__ Near2 hctSeries2(float2 r, float2 invr, float2 rho, f
   if (FAR) {
     return Near2{false, false};
   }
-  // written so that a distance that is not a number is left to the closed forms, as before
+  // written so that a distance that is not a number (r = 0) is left to the closed forms, which add
+  // nothing there
   return Near2{!(r.x > touch.x && t.x <= kSeriesLimit), !(r.y > touch.y && t.y <= kSeriesLimit)};
 }
 
@@ -1259,10 +1260,11 @@ struct RadiiPass {
       }
     }
     late |= (late_x ? bit : 0u) | (late_y ? bit << 16 : 0u);
-    const float2 keep = f2(late_x ? 0.0f : (GUARD ? -wt.x : -1.0f),
-                           late_y ? 0.0f : (GUARD ? -wt.y : -1.0f));
-    psi_i = fma2(hi, keep, psi_i);
-    psi_j = fma2(hj, keep, psi_j);
+    // a select, not a weight of zero: the series grows as r^-20 and overflows where two atoms
+    // nearly coincide (below 0.015 A for a screened radius of 1.4), and zero times that is NaN
+    const float2 neg = GUARD ? f2(-wt.x, -wt.y) : f2(-1.0f);
+    psi_i = fma2(f2(late_x ? 0.0f : hi.x, late_y ? 0.0f : hi.y), neg, psi_i);
+    psi_j = fma2(f2(late_x ? 0.0f : hj.x, late_y ? 0.0f : hj.y), neg, psi_j);
     if (STORE) {
       __stcg(out, make_float4(di.x, di.y, dj.x, dj.y));
     }
