@@ -254,7 +254,7 @@ struct Radii64 {
       const double dx = c.x - a.x, dy = c.y - a.y, dz = c.z - a.z;
       const double r2 = dx * dx + dy * dy + dz * dz;
       const double invr = rsqrt(r2);
-      const double r = r2 * invr;
+      const double r = sqrt(r2);          // 0 for coincident atoms, where r2 * invr is no number
       double hi = hctIntegral64(r, r2, invr, b.x, b.z, c.w);
       double hj = hctIntegral64(r, r2, invr, d.x, d.z, a.w);
       if (neck.size > 0 && r < b.x + d.x + neck.reach) {

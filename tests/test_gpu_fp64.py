@@ -171,3 +171,28 @@ def test_fp64_mode_minimization_follows_the_oracle(clash_cycles):
         assert rel64[:10].max() <= 1e-8, (k, rel64[:10].max())
         assert abs(hist[k, -1] - h_ref[-1]) <= 1e-6 * drop, k
         assert rel64.max() <= rel32.max(), k
+
+
+def test_coincident_atoms_take_the_neck_term():
+    """Two atoms at one point, neither's screened radius above the other's offset radius, descreen
+    each other by the neck term alone, the limit of a small distance: the oracle at 1e-6 A, where
+    psi differs by less than 1e-6 times its slope there (below 1 per A).  The workspace's grid is
+    2^-24."""
+    g = load("synthetic_N8.npz")
+    mol = molecule_from_fixture(g)
+    rho = np.asarray(mol.pb_radii) - 0.195141
+    s = np.asarray(mol.gb_screen) * rho
+    a, b = next((i, j) for i in range(mol.natom) for j in mol.excl12[i]
+                if i < j and rho[i] >= s[j] and rho[j] >= s[i])
+    xyz = _on_grid(mol.coords)
+    xyz[b] = xyz[a]
+    near = xyz.copy()
+    near[b] += [1.0e-6, 0.0, 0.0]
+    ref = oracle.from_fixture(g).evaluate(near)["psi"]
+    syn = sb.Synthesis([mol], precision=sb.PRECISION_DOUBLE, **solvent_options(g))
+    syn.set_coordinates(xyz)
+    syn.initialize()
+    syn.evaluate(terms=sb.TERM_GB, force=False)
+    psi = syn.gb_workspace()[0]
+    assert np.abs(psi - ref)[[a, b]].max() <= 1.0e-6 + 2.0 ** -24
+    syn.close()
