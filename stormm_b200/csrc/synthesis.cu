@@ -83,6 +83,7 @@ const char* lastError() { return g_last_error.c_str(); }
 
 void cudaCheck(cudaError_t err, const char* what) {
   if (err != cudaSuccess) {
+    cudaGetLastError();   // reported here, not left for the next launch check to find
     throw Error(SB_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(err));
   }
 }

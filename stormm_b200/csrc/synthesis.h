@@ -68,6 +68,8 @@ template <typename T> struct DeviceArray {
       }
     }
     p = nullptr;
+    n = 0;
+    s = nullptr;
     owned = true;
   }
   void view(T* ptr, size_t count) {
@@ -76,19 +78,22 @@ template <typename T> struct DeviceArray {
     n = count;
     owned = false;
   }
+  // n holds only once the memory does: an allocation that fails leaves the array empty, so that
+  // callers who keep an array while it is large enough allocate again
   void allocate(size_t count) {
     release();
-    n = count;
-    s = allocationStream();
+    const cudaStream_t on = allocationStream();
     const size_t bytes = sizeof(T) * (count > 0 ? count : 1);
-    if (s != nullptr) {
-      cudaCheck(cudaMallocAsync(reinterpret_cast<void**>(&p), bytes, s), "cudaMallocAsync");
+    if (on != nullptr) {
+      cudaCheck(cudaMallocAsync(reinterpret_cast<void**>(&p), bytes, on), "cudaMallocAsync");
+      s = on;
       // usable by the synchronous copies that follow
-      cudaCheck(cudaStreamSynchronize(s), "cudaMallocAsync");
+      cudaCheck(cudaStreamSynchronize(on), "cudaMallocAsync");
     }
     else {
       cudaCheck(cudaMalloc(reinterpret_cast<void**>(&p), bytes), "cudaMalloc");
     }
+    n = count;
   }
   void zeros(size_t count) {
     allocate(count);
