@@ -901,6 +901,7 @@ std::unique_ptr<UnitPlan> Synthesis::makePlan(int max_slots_cap, int max_tiles_c
     }
     systems.push_back(s);
     plan->small_tiles += tiles_of(s);
+    plan->small_widest = std::max(plan->small_widest, slots_of(s));
     cur.y++;
     cur.z += slots_of(s);
     cur.w += tiles_of(s);
@@ -1061,12 +1062,17 @@ void Synthesis::buildUnits() {
   if (opt.max_tiles_per_unit > 0) tiles_cap = opt.max_tiles_per_unit;
   eval_plan = makePlan(slots_cap, tiles_cap, true);
   // Minimization keeps whole molecules on chip for hundreds of cycles.  A batch of at most one
-  // molecule per SM gives each its own block, in one launch and with 512 threads (launchMinPlan):
-  // such a launch lasts as long as its largest molecule.  128 molecules of 12-512 atoms, 60 cycles:
-  // one launch after another with 256 threads 16.8 ms, this way 8.3 ms.  Larger batches share units
-  // of up to 128 slots, which balance the persistent grid (sb_autotune can choose another packing).
-  min_plan = (nfused <= sm_count) ? makePlan(std::max(widest, kTile), 1, true) :
-                                    makePlan(128, 16, true);
+  // molecule per SM gives each its own block, in one launch: such a launch lasts as long as its
+  // largest molecule.  128 molecules of 12-512 atoms, 60 cycles: one launch after another with 256
+  // threads 16.8 ms, this way 8.3 ms.  Larger batches share units of up to 128 slots, which balance
+  // the persistent grid (sb_autotune can choose another packing), and so do those of molecules of
+  // up to 64 atoms unless sixteen such batches (the request server's most in flight) fit on the GPU
+  // at once: the blocks of several small batches would wait for each other.  50 cycles, one batch of
+  // 64 / sixteen batches of 64 on their own streams, molecules of 20 atoms: a block each 2.6 / 10.8
+  // ms, shared units 3.2 / 3.7; of 64 atoms 3.0 / 13.3 and 3.9 / 10.1; of 96 atoms 3.7 / 19.1 and
+  // no different, a unit holding one of those.
+  const bool share = nfused > sm_count || (widest <= 64 && nfused > sm_count / 8);
+  min_plan = share ? makePlan(128, 16, true) : makePlan(std::max(widest, kTile), 1, true);
   // one unit per system, in system order, for the per-system launches
   auto slots_of = [&](int s) { return (atom_count[s] + kTile - 1) / kTile * kTile; };
   auto tiles_of = [&](int s) {
@@ -1878,6 +1884,21 @@ void Synthesis::checkMinimizeSmem(int slots, int lj) const {
   }
 }
 
+// Threads a block for an on-chip minimization launch of `units` units, whose largest molecule takes
+// `widest` atom slots: 512 for at most a unit per SM, if that molecule has ten tiles or more (50
+// cycles of 100 molecules of 128 atoms 3.9 ms against 5.2 with 256 threads, of 96 atoms 3.5 against
+// 3.7) or the batch is so small that sixteen of them (the request server's most in flight) find an
+// SM for each unit.  A 512-thread block fills an SM's registers, so that several small batches at
+// once wait for each other: four batches of 64 molecules of 20 atoms 5.4 ms against 2.8 with 256
+// threads, of 24-96 atoms 6.1 against 4.8; of 128 atoms 7.9 against 8.1.  A molecule of one tile
+// has no work for more than 256 threads.
+int Synthesis::minimizeThreads(int units, int widest) const {
+  if (opt.threads_per_block > 0 || units > sm_count) {
+    return threads;
+  }
+  return (widest > 96 || (widest > kTile && 16 * units <= sm_count)) ? 512 : threads;
+}
+
 void Synthesis::launchMinPlan(const UnitPlan &plan, int cycles, bool final_energy,
                               cudaStream_t stream) {
   DevMinimizer m = dev_min;
@@ -1898,10 +1919,9 @@ void Synthesis::launchMinPlan(const UnitPlan &plan, int cycles, bool final_energ
     d.max_unit_slots = plan.small_slots;
     m.queue = d_queue.p + 1;
     checkMinimizeSmem(plan.small_slots, plan.small_lj);
-    // a block per SM at most: twice the warps on each unit
-    const int wide = (opt.threads_per_block <= 0 && nunit - plan.n_big <= sm_count) ? 512 : threads;
     cudaCheck(launchMinimize(d, m, plan.n_big, nunit, plan.small_lj, cycles, final_energy,
-                             wide, sm_count, stream), "minimization launch");
+                             minimizeThreads(nunit - plan.n_big, plan.small_widest), sm_count,
+                             stream), "minimization launch");
   }
 }
 

@@ -170,6 +170,7 @@ struct UnitPlan {
   int big_slots = 0, big_lj = 0;
   int small_slots = 0, small_lj = 0;
   long long big_tiles = 0, small_tiles = 0;
+  int small_widest = 0;          // atom slots of the largest molecule in the packed units
   std::vector<int> meta;         // kUnitMetaFields ints per molecule row, plus a closing row
   std::vector<int4> desc;        // as units, but x = first row of the unit in meta
   DeviceArray<int4> d_units;     // desc on the device
@@ -216,6 +217,7 @@ public:
   void downloadResults(double* forces, double* energies, cudaStream_t stream);
   void setRestraints(const sb_restraint* list, int count);
   int launchThreads(int units, int slots, long long tiles, int terms) const;
+  int minimizeThreads(int units, int widest) const;
   void getEnergiesFixed(long long* out, cudaStream_t stream);
   void getGbWorkspace(double* psi, double* radii, double* sde, cudaStream_t stream);
   int checkStatus(cudaStream_t stream);

@@ -54,19 +54,68 @@ def test_packing_and_block_size_rules_change_no_bit(count, threads):
 @pytest.mark.gpu
 def test_on_chip_minimizer_block_size_changes_no_bit():
     """148 molecules take a 512-thread block each, 149 share units of 256-thread blocks."""
+    _minimized_alike((20, 40, 130, 300), 148, 149)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sizes,few,many", [((17, 24, 32), 18, 19), ((17, 40, 64), 18, 19),
+                                            ((17, 40, 96), 9, 10), ((40, 96, 97), 10, 10)])
+def test_on_chip_minimizer_rules_change_no_bit(sizes, few, many):
+    """Small molecules on both sides of the lines between a block each and shared units, and
+    between 512 and 256 threads (148 SMs), with the same molecules in 256-thread blocks."""
+    _minimized_alike(sizes, few, many)
+
+
+def _minimized_alike(sizes, few, many):
     import stormm_b200 as sb
     from stormm_b200 import synthetic
-    mols = [synthetic.make_molecule(800 + k, n) for k, n in enumerate((20, 40, 130, 300))]
+    mols = [synthetic.make_molecule(800 + k, n) for k, n in enumerate(sizes)]
     final = []
-    for count in (148, 149):
+    for count, opts in ((few, {}), (many, {}), (many, dict(threads_per_block=256))):
         index = np.arange(count, dtype=np.int32) % len(mols)
-        syn = sb.Synthesis(mols, topology_index=index)
+        syn = sb.Synthesis(mols, topology_index=index, **opts)
         syn.set_coordinates(np.concatenate([mols[t].coords for t in index]))
         syn.minimize(total_cycles=12, sd_cycles=4, kernel=sb.MIN_PERSISTENT)
-        final.append(syn.split(syn.coordinates())[:148])
+        final.append(syn.split(syn.coordinates())[:few])
         syn.close()
-    for a, b in zip(*final):
+    for a, b, c in zip(*final):
         assert np.array_equal(a, b)
+        assert np.array_equal(a, c)
+
+
+@pytest.mark.gpu
+def test_small_on_chip_batches_share_the_gpu():
+    """Four batches of 64 small molecules on their own streams take little longer than one: with a
+    512-thread block a molecule they waited for each other and took 2.1 times as long."""
+    import time
+
+    import torch
+    import stormm_b200 as sb
+    from stormm_b200 import synthetic
+    mol = synthetic.make_molecule(850, 20)
+    index = np.zeros(64, dtype=np.int32)
+    xyz = np.concatenate([mol.coords] * 64)
+    syns = [sb.Synthesis([mol], topology_index=index) for _ in range(4)]
+    streams = [torch.cuda.Stream() for _ in syns]
+
+    def seconds(count):
+        best = 1.0e9
+        for _ in range(6):
+            for syn in syns[:count]:
+                syn.set_coordinates(xyz)
+            torch.cuda.synchronize()
+            t0 = time.perf_counter()
+            for syn, stream in zip(syns[:count], streams):
+                syn.minimize(stream=stream.cuda_stream, total_cycles=100, sd_cycles=20,
+                             kernel=sb.MIN_PERSISTENT)
+            torch.cuda.synchronize()
+            best = min(best, time.perf_counter() - t0)
+        return best
+
+    one, four = seconds(1), seconds(4)
+    assert four <= 1.5 * one, (one, four)
+    for syn in syns:
+        syn.close()
 
 
 @pytest.mark.gpu
