@@ -1060,6 +1060,7 @@ void Synthesis::buildUnits() {
   }
   if (opt.max_atoms_per_unit > 0) slots_cap = opt.max_atoms_per_unit;
   if (opt.max_tiles_per_unit > 0) tiles_cap = opt.max_tiles_per_unit;
+  eval_caps = std::make_pair(slots_cap, tiles_cap);
   eval_plan = makePlan(slots_cap, tiles_cap, true);
   // Minimization keeps whole molecules on chip for hundreds of cycles.  A batch of at most one
   // molecule per SM gives each its own block, in one launch: such a launch lasts as long as its
@@ -1072,7 +1073,8 @@ void Synthesis::buildUnits() {
   // ms, shared units 3.2 / 3.7; of 64 atoms 3.0 / 13.3 and 3.9 / 10.1; of 96 atoms 3.7 / 19.1 and
   // no different, a unit holding one of those.
   const bool share = nfused > sm_count || (widest <= 64 && nfused > sm_count / 8);
-  min_plan = share ? makePlan(128, 16, true) : makePlan(std::max(widest, kTile), 1, true);
+  min_caps = share ? std::make_pair(128, 16) : std::make_pair(std::max(widest, kTile), 1);
+  min_plan = makePlan(min_caps.first, min_caps.second, true);
   // one unit per system, in system order, for the per-system launches
   auto slots_of = [&](int s) { return (atom_count[s] + kTile - 1) / kTile * kTile; };
   auto tiles_of = [&](int s) {
@@ -2054,6 +2056,13 @@ void Synthesis::autotune(int what, int* chosen_slots, int* chosen_tiles, double*
   for (const auto &c : kFixed) {
     candidates.emplace_back(c[0], c[1]);
   }
+  auto consider = [&](const std::pair<int, int> &c) {
+    if (std::find(candidates.begin(), candidates.end(), c) == candidates.end()) {
+      candidates.push_back(c);
+    }
+  };
+  // the default packing, which the fixed ones need not hold
+  consider((what == SB_TUNE_EVALUATE) ? eval_caps : min_caps);
   if (what == SB_TUNE_EVALUATE) {
     // Wave-sized packings: tile caps that split the fused tiles into one to four waves of the
     // evaluation kernel's resident blocks (four per SM), so the last wave is not a sliver
@@ -2068,10 +2077,7 @@ void Synthesis::autotune(int what, int* chosen_slots, int* chosen_tiles, double*
     for (int waves = 1; waves <= 4; waves++) {
       const long long cap = (tiles_all + waves * resident - 1) / (waves * resident);
       if (cap >= 6 && cap <= 64) {
-        const std::pair<int, int> c(256, static_cast<int>(cap));
-        if (std::find(candidates.begin(), candidates.end(), c) == candidates.end()) {
-          candidates.push_back(c);
-        }
+        consider(std::make_pair(256, static_cast<int>(cap)));
       }
     }
   }
@@ -2107,8 +2113,8 @@ void Synthesis::autotune(int what, int* chosen_slots, int* chosen_tiles, double*
     catch (const Error &) {
       continue;   // a candidate that does not fit this synthesis
     }
-    // evaluation packings are timed with both block-size rules: 512-thread blocks for launches
-    // of fewer units than one wave of 256-thread blocks, or 256 threads throughout
+    // evaluation packings are timed with both block-size rules, launchThreads() by units, slots and
+    // tiles or 256 threads throughout; minimizer packings with the threads of minimizeThreads()
     const int modes = (what == SB_TUNE_EVALUATE && opt.threads_per_block <= 0) ? 2 : 1;
     double plan_best = 1.0e30;
     bool plan_wide = keep_wide;
@@ -2125,6 +2131,8 @@ void Synthesis::autotune(int what, int* chosen_slots, int* chosen_tiles, double*
       }
       else {
         minimizeBegin(ctl, stream);
+        // no cycles: a kernel's first launch loads it, which is no part of its time
+        launchMinPlan(*plan, 0, false, stream);
         cudaCheck(cudaEventRecord(e0, stream), "cudaEventRecord");
         launchMinPlan(*plan, ctl.total_cycles, false, stream);
         cudaCheck(cudaEventRecord(e1, stream), "cudaEventRecord");

@@ -387,7 +387,8 @@ private:
   std::unique_ptr<UnitPlan> makePlan(int max_slots_cap, int max_tiles_cap,
                                      bool defer = false) const;
   void finalizePlan(UnitPlan* plan, bool defer = false) const;
-  bool allow_wide = true;        // 512-thread blocks for small all-term launches (autotuned)
+  bool allow_wide = true;        // block sizes by launchThreads(), or `threads` alone (autotuned)
+  std::pair<int, int> eval_caps, min_caps;   // slot and tile caps of the default plans
   void launchPlan(const UnitPlan &plan, int terms, bool force, bool energy, cudaStream_t stream,
                   const Clash &clash = Clash());
   void checkMinimizeSmem(int slots, int lj) const;

@@ -119,6 +119,42 @@ def test_small_on_chip_batches_share_the_gpu():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("lo,hi", [(12, 512), (300, 500)])
+def test_tuned_minimizer_keeps_up_with_the_default(lo, hi):
+    """128 molecules with some above 256 atoms, which the default puts in one launch: the packing
+    that sb_autotune keeps was 1.3 to 1.6 times as slow while the default was no candidate."""
+    import torch
+    import stormm_b200 as sb
+    from stormm_b200 import synthetic
+    sizes = np.random.default_rng(9).integers(lo, hi + 1, size=32)
+    mols = [synthetic.make_molecule(870 + k, int(n)) for k, n in enumerate(sizes)]
+    index = np.arange(128, dtype=np.int32) % len(mols)
+    xyz = np.concatenate([mols[t].coords for t in index])
+
+    def milliseconds(syn):
+        best = 1.0e9
+        for _ in range(4):
+            syn.set_coordinates(xyz)
+            torch.cuda.synchronize()
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            syn.minimize(total_cycles=12, sd_cycles=4, kernel=sb.MIN_PERSISTENT)
+            b.record()
+            torch.cuda.synchronize()
+            best = min(best, a.elapsed_time(b))
+        return best
+
+    tuned = sb.Synthesis(mols, topology_index=index)
+    tuned.set_coordinates(xyz)
+    tuned.autotune(sb.TUNE_MINIMIZE)
+    plain = sb.Synthesis(mols, topology_index=index)
+    t, d = milliseconds(tuned), milliseconds(plain)
+    assert t <= 1.15 * d, (t, d)
+    tuned.close()
+    plain.close()
+
+
+@pytest.mark.gpu
 def test_widest_blocks_change_no_bit():
     """148 molecules of sixteen tiles and more take 1,024-thread blocks, 149 of them 512."""
     import stormm_b200 as sb
