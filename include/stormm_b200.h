@@ -241,9 +241,9 @@ int sb_evaluate_clash(sb_synthesis* syn, int terms, int eval_force, int eval_ene
                       double clash_distance, double clash_ratio, void* stream);
 
 /* Number of work units the batched launches use, and the launch shape chosen: threads is the
- * block size of the evaluation launch of packed units (512 when that launch holds fewer units
- * than one wave of 256-thread blocks, unless sb_autotune found 256 faster or threads_per_block
- * fixes it) */
+ * block size of the evaluation launch of packed units: 128, 256, 512 or 1,024 by the number of
+ * units, their atom slots and their tiles (fewer units, more threads), 256 throughout where
+ * sb_autotune found that faster, or what threads_per_block fixes */
 int sb_launch_info(const sb_synthesis* syn, int* work_units, int* blocks, int* threads);
 
 /* ------------------------------------------------------------------------------------------ */

@@ -33,13 +33,14 @@ constexpr int kDeijdaBits = 23;           // fixed-point bits of the in-block dE
 // Fields of a unit molecule's row: everything a block needs to know of its molecules, so that no
 // step of an evaluation waits on a chain of loads through the per-system arrays
 enum UnitMetaField : int {
-  kMetaSystem = 0, kMetaAtoms, kMetaSlot, kMetaTile, kMetaLj,    // system, atoms; first slot, tile
-                                                                 // and table entry in the unit
-  kMetaBondChunk, kMetaAnglChunk, kMetaDiheChunk,                // first chunks of 32 terms
-  kMetaAtom0, kMetaMask0, kMetaLjTable, kMetaTypes,              // atom_start, tile_start, lj_start;
-                                                                 // types | terms in the last bond,
-                                                                 // angle, dihedral chunk << 8, 14, 20
-  kMetaBond0, kMetaAngl0, kMetaDihe0                             // bond_start, angl_start, dihe_start
+  kMetaSystem = 0, kMetaAtoms, kMetaSlot, kMetaTile, kMetaLj,   // system, atoms; first slot, tile
+                                                                // and table entry in the unit
+  kMetaBondChunk, kMetaAnglChunk, kMetaDiheChunk,               // first chunks of 32 terms
+  kMetaAtom0, kMetaMask0, kMetaLjTable, kMetaTypes,             // atom_start, tile_start, lj_start;
+                                                                // types | terms in the last bond <<
+                                                                // 8, angle << 14, dihedral chunk
+                                                                // << 20
+  kMetaBond0, kMetaAngl0, kMetaDihe0                            // bond_, angl_ and dihe_start
 };
 
 // Energy slots (Potential/energy_enumerators.h:36-50)

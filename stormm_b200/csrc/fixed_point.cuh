@@ -48,17 +48,11 @@ __device__ __forceinline__ void atomicAddInt63(float v, int* primary, int* overf
 // and for two atoms both hi_j - hi_i and lo_j - lo_i are exact in FP32 (hi differences are below
 // 2^24 units of 2^-10, lo differences below 2^22 units of 2^-32), so their sum rounds the exact
 // separation once and that rounding's error is lo_d - (d - hi_d), recoverable in two additions
-// (separationError).  An unconstrained hi = (float)x loses both properties.
+// (PairPass).  An unconstrained hi = (float)x loses both properties.
 __device__ __forceinline__ void splitCoordinate(double x, float* hi, float* lo) {
   const double h = rint(x * 1024.0) * 0.0009765625;
   *hi = static_cast<float>(h);
   *lo = static_cast<float>(x - h);
-}
-
-// Rounding error of d = hd + ld, where hd and ld are separations of hi and lo parts from
-// splitCoordinate: the exact separation is d + separationError(hd, ld, d)
-__device__ __forceinline__ float separationError(float hd, float ld, float d) {
-  return __fsub_rn(ld, __fsub_rn(d, hd));
 }
 
 // int63 pair -> int64

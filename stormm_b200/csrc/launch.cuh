@@ -6,12 +6,15 @@
 // one before it before it ends, the order of the whole chain is kept.  After a kernel or a copy
 // that gives no such signal the launch is an ordinary one.
 //
-// Taken by the tiled path, whose evaluation of one chain is eight short kernels in a row, and by the
-// clearing and conversion kernels (one 2,500-atom chain with copies 116 -> 98 us; 1,024 molecules,
-// through the latter alone, 389 -> 380).  Not by the fused evaluation, whose large units come first
-// and are then placed on the SMs that happen to be free (1,024 molecules 389 -> 436 us), the FP64
-// passes (128 molecules 206 -> 216) or the minimizer's cycle graph (one molecule, 60 cycles 4.38 ->
-// 4.59 ms).
+// Taken by the tiled path, whose evaluation of one chain is eight short kernels in a row, and by
+// the clearing and conversion kernels (one 2,500-atom chain with copies 116 -> 98 us; 1,024
+// molecules, through the latter alone, 389 -> 380).  Not by the fused evaluation, whose large units
+// come first and are then placed on the SMs that happen to be free (1,024 molecules 389 -> 436 us),
+// the FP64 passes (128 molecules 206 -> 216) or the line-search kernels.  The graph minimizer's
+// captured cycle begins with the clearing kernel, to which nothing in the graph is a predecessor,
+// and holds the tiled passes of molecules on the tiled path as programmatic edges; its fused
+// evaluations and line-search steps are ordinary nodes (all of them launched this way: one
+// molecule, 60 cycles 4.38 -> 4.59 ms).
 #ifndef STORMM_B200_LAUNCH_CUH
 #define STORMM_B200_LAUNCH_CUH
 

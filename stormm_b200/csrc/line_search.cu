@@ -50,7 +50,7 @@ __device__ __forceinline__ int firstWarp() {
 
 __device__ __forceinline__ int warpStride() { return (gridDim.x * blockDim.x) >> 5; }
 
-// A system's line-search scalars, one per lane, fetched by one load; field() hands one to every lane
+// A system's line-search scalars, one per lane, fetched by one load; field() hands one to all lanes
 struct LineScalars {
   double mine;
   __device__ __forceinline__ LineScalars(const double* line, int lane) :

@@ -434,7 +434,8 @@ __global__ void kMinimizerReset(DevMinimizer m, int nsys, int natom_padded, doub
 }  // namespace
 
 size_t minimizeSmemBytes(int max_slots, int max_lj, int threads) {
-  return unitSmemBytes(max_slots, max_lj, threads) + minSmemBytes(max_slots, unitSystems(max_slots));
+  return unitSmemBytes(max_slots, max_lj, threads) +
+         minSmemBytes(max_slots, unitSystems(max_slots));
 }
 
 

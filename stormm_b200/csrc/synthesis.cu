@@ -1046,10 +1046,10 @@ void Synthesis::buildUnits() {
   // share a unit, larger ones run alone (1,024 molecules of 16-256 atoms: 213 us against 238 us for
   // units packed up to 36 tiles, which leave a sliver of a second wave).  All molecules of up to
   // 128 atoms: one a unit while that is one wave of 256-thread blocks (512 molecules of 24-96 atoms
-  // 44 us, four tiles a unit 52), and again beyond 1.25 waves, where launchThreads() takes 128-thread
-  // blocks (1,024 molecules: 71 us, four tiles a unit in 256-thread blocks 81); from two waves of
-  // those on, units of up to eight tiles if the molecules average fewer than five (4,096 molecules:
-  // 253 us, one a unit 260, four tiles a unit in 256-thread blocks 293).
+  // 44 us, four tiles a unit 52), and again beyond 1.25 waves, where launchThreads() takes
+  // 128-thread blocks (1,024 molecules: 71 us, four tiles a unit in 256-thread blocks 81); from two
+  // waves of those on, units of up to eight tiles if the molecules average fewer than five (4,096
+  // molecules: 253 us, one a unit 260, four tiles a unit in 256-thread blocks 293).
   int slots_cap = 256, tiles_cap = 4;
   if (widest <= 128 && nfused <= 4 * sm_count) {
     tiles_cap = 1;
@@ -1068,10 +1068,10 @@ void Synthesis::buildUnits() {
   // threads 16.8 ms, this way 8.3 ms.  Larger batches share units of up to 128 slots, which balance
   // the persistent grid (sb_autotune can choose another packing), and so do those of molecules of
   // up to 64 atoms unless sixteen such batches (the request server's most in flight) fit on the GPU
-  // at once: the blocks of several small batches would wait for each other.  50 cycles, one batch of
-  // 64 / sixteen batches of 64 on their own streams, molecules of 20 atoms: a block each 2.6 / 10.8
-  // ms, shared units 3.2 / 3.7; of 64 atoms 3.0 / 13.3 and 3.9 / 10.1; of 96 atoms 3.7 / 19.1 and
-  // no different, a unit holding one of those.
+  // at once: the blocks of several small batches would wait for each other.  50 cycles, one batch
+  // of 64 / sixteen batches of 64 on their own streams, molecules of 20 atoms: a block each 2.6 /
+  // 10.8 ms, shared units 3.2 / 3.7; of 64 atoms 3.0 / 13.3 and 3.9 / 10.1; of 96 atoms 3.7 / 19.1
+  // and no different, a unit holding one of those.
   const bool share = nfused > sm_count || (widest <= 64 && nfused > sm_count / 8);
   min_caps = share ? std::make_pair(128, 16) : std::make_pair(std::max(widest, kTile), 1);
   min_plan = makePlan(min_caps.first, min_caps.second, true);

@@ -75,10 +75,11 @@ __device__ __forceinline__ int tiledAtom(const DevSynthesis &d, const DevTiled &
 }
 
 // Blocks for a tile pass.  Each warp takes `per` tiles one after another, a serial chain: one
-// tile a warp while the tiles make fewer than four waves of resident warps (four blocks of eight
-// an SM), so that a single chain or a small FP64 batch spreads over every SM, and up to eight
-// beyond that, which keeps the energy flushes (once per molecule and run of tiles) rare while the
-// block scheduler still balances a few waves.  Sums are integers, so the split changes no bit.
+// tile a warp below eight waves (a wave: four blocks of eight warps an SM, though the passes of
+// more registers keep three resident), so that a single chain or a small FP64 batch spreads over
+// every SM, then a quarter of the waves, up to eight tiles from 32 waves on, which keeps the energy
+// flushes (once per molecule and run of tiles) rare while the block scheduler still balances four
+// waves or more.  Sums are integers, so the split changes no bit.
 // Against a fixed four tiles a warp: one 2,500-atom chain (3,160 tiles), pass 1 / 2 / 3 31 / 41 /
 // 38 us -> 18 / 24 / 20; 128 small molecules in FP64 (2,043 tiles) 163 / 136 / 162 us -> 64 / 47 /
 // 65; 32 chains (200,000 tiles) 434 / 792 / 499 us -> 424 / 780 / 479.

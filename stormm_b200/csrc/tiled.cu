@@ -4,13 +4,13 @@
 // contract a few operations differently in the two kernels) and each is bit-identical from run
 // to run.
 //
-// Every 32 x 32 tile of every tiled molecule is a warp task.  kTiledPrepare lays the atoms out as
-// pair records (coordinates as hi / lo float pairs, the passes' payloads); a warp copies the tile's
-// two blocks of records into its own slice of shared memory, walks the tile with the fused kernel's functors, and adds its accumulators to global
-// integer arrays.  Passes that need the whole molecule finished first (effective radii after
-// pass 1, the chain-rule prefactor after pass 2) are separate per-atom kernels.  Warps take
-// contiguous runs of tiles, so a warp's energy sums change molecule rarely and flush once per
-// molecule.
+// Every 32 x 32 tile of every tiled molecule is a warp task. kTiledPrepare lays the atoms out as
+// pair records (coordinates as hi / lo float pairs, the passes' payloads); a warp copies the
+// tile's two blocks of records into its own slice of shared memory, walks the tile with the fused
+// kernel's functors, and adds its accumulators to global integer arrays. Passes that need the
+// whole molecule finished first (effective radii after pass 1, the chain-rule prefactor after pass
+// 2) are separate per-atom kernels. Warps take contiguous runs of tiles, so a warp's energy sums
+// change molecule rarely and flush once per molecule.
 #include <cuda_runtime.h>
 
 #include "launch.cuh"
@@ -185,7 +185,8 @@ kTiledPrepare(const DevSynthesis d, const DevTiled t, int atom_begin, int atom_e
 // near forms of the descreening (4 times the screened radius, overlapping spheres, the neck)
 constexpr float kPlainDistance = 10.0f;
 
-__device__ __forceinline__ bool tilePlain(const DevSynthesis &d, const DevTiled &t, int ia, int ja) {
+__device__ __forceinline__ bool tilePlain(const DevSynthesis &d, const DevTiled &t, int ia,
+                                          int ja) {
   const float4 ci = t.boxes[2 * (ia / kTile)], hi = t.boxes[2 * (ia / kTile) + 1];
   const float4 cj = t.boxes[2 * (ja / kTile)], hj = t.boxes[2 * (ja / kTile) + 1];
   const float gx = fmaxf(fabsf(ci.x - cj.x) - hi.x - hj.x, 0.0f);
@@ -542,13 +543,16 @@ cudaError_t launchTiled(const DevSynthesis &d, const DevTiled &t, const int* h_t
     int vrows = 2 * sm_count / nmol;
     vrows = vrows < 4 ? 4 : (vrows > 32 ? 32 : vrows);
     const dim3 vgrid(nmol, vrows);
+#define SB_VALE_GO(F, E, C)                                                                    \
+    launchAfter(kTiledValence<F, E, C>, vgrid, 256, 0, stream, d, t, mol_begin);
 #define SB_VALE(C)                                                                             \
-    if (force && energy) launchAfter(kTiledValence<true, true, C>, vgrid, 256, 0, stream, d, t, mol_begin); \
-    else if (force) launchAfter(kTiledValence<true, false, C>, vgrid, 256, 0, stream, d, t, mol_begin);   \
-    else launchAfter(kTiledValence<false, true, C>, vgrid, 256, 0, stream, d, t, mol_begin);
+    if (force && energy) SB_VALE_GO(true, true, C)                                             \
+    else if (force) SB_VALE_GO(true, false, C)                                                 \
+    else SB_VALE_GO(false, true, C)
     if (clash) { SB_VALE(true) }
     else { SB_VALE(false) }
 #undef SB_VALE
+#undef SB_VALE_GO
   }
   if (nb || gb) {
     launchAfter(kTiledPrepare, agrid, 256, 0, stream, d, t, ab, ae);
@@ -565,10 +569,12 @@ cudaError_t launchTiled(const DevSynthesis &d, const DevTiled &t, const int* h_t
 #undef SB_ATOMS
   }
   if (nb || gb) {
+#define SB_PAIR_GO(F, E, NB, GB, C)                                                           \
+    launchAfter(kTiledPair<F, E, NB, GB, C>, tgrid, 256, 0, stream, d, t, tb, te);
 #define SB_PAIR(F, E, C)                                                                      \
-    if (nb && gb) launchAfter(kTiledPair<F, E, true, true, C>, tgrid, 256, 0, stream, d, t, tb, te);    \
-    else if (nb) launchAfter(kTiledPair<F, E, true, false, C>, tgrid, 256, 0, stream, d, t, tb, te);   \
-    else launchAfter(kTiledPair<F, E, false, true, false>, tgrid, 256, 0, stream, d, t, tb, te);
+    if (nb && gb) SB_PAIR_GO(F, E, true, true, C)                                             \
+    else if (nb) SB_PAIR_GO(F, E, true, false, C)                                             \
+    else SB_PAIR_GO(F, E, false, true, false)
     if (clash) {
       if (force && energy) { SB_PAIR(true, true, true) }
       else if (force) { SB_PAIR(true, false, true) }
@@ -580,6 +586,7 @@ cudaError_t launchTiled(const DevSynthesis &d, const DevTiled &t, const int* h_t
       else { SB_PAIR(false, true, false) }
     }
 #undef SB_PAIR
+#undef SB_PAIR_GO
   }
   if (gb && force) {
     if (workspace) launchAfter(kTiledChain<true>, agrid, 256, 0, stream, d, t, ab, ae);

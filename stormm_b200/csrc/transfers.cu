@@ -102,8 +102,8 @@ cudaError_t launchImportCoordinates(const double* d_xyz, const int* d_map, int n
                                     double scale, long long* xcrd, long long* ycrd,
                                     long long* zcrd, int* xo, int* yo, int* zo, int* status,
                                     cudaStream_t stream) {
-  launchAfter(kImportCoordinates, gridFor(natom), 256, 0, stream, d_xyz, d_map, natom, scale, xcrd, ycrd,
-                                                         zcrd, xo, yo, zo, status);
+  launchAfter(kImportCoordinates, gridFor(natom), 256, 0, stream, d_xyz, d_map, natom, scale,
+              xcrd, ycrd, zcrd, xo, yo, zo, status);
   return cudaGetLastError();
 }
 
@@ -111,7 +111,7 @@ cudaError_t launchExportCoordinates(const long long* xcrd, const long long* ycrd
                                     const long long* zcrd, const int* d_map, int natom,
                                     double inv_scale, double* d_xyz, cudaStream_t stream) {
   launchAfter(kExportCoordinates, gridFor(natom), 256, 0, stream, xcrd, ycrd, zcrd, d_map, natom,
-                                                         inv_scale, d_xyz);
+              inv_scale, d_xyz);
   return cudaGetLastError();
 }
 
@@ -119,7 +119,7 @@ cudaError_t launchExportForces(const long long* xf, const long long* yf, const l
                                const int* xo, const int* yo, const int* zo, const int* d_map,
                                int natom, double inv_scale, double* d_xyz, cudaStream_t stream) {
   launchAfter(kExportForces, gridFor(natom), 256, 0, stream, xf, yf, zf, xo, yo, zo, d_map, natom,
-                                                    inv_scale, d_xyz);
+              inv_scale, d_xyz);
   return cudaGetLastError();
 }
 

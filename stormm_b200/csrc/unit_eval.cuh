@@ -33,11 +33,11 @@
 // with its copies, 445 -> 391 us; 60 minimization cycles of 4,096 molecules of 24-96 atoms 61.5 ->
 // 50.7 ms; 32 chains of 2,000-5,000 atoms 1,817 -> 1,600 us.
 //
-// Shared memory per atom pair record: pa = (x, x', y, y'), pb = (z, z', w1, w1'), pc = (lo x, lo x',
-// lo y, lo y'), pd = (lo z, lo z', w2, w2') and pg = (g, g', h, h'), where w1 / w2 carry what the
-// pass needs (pass 1 and 3: s*rho and rho; pass 2: charge and effective radius), g the reciprocal
-// effective radius and h the Lennard-Jones code bits (pass 2) or the chain-rule dE/dR (pass 3).
-// prm holds the static per-atom values.
+// Shared memory per atom pair record: pa = (x, x', y, y'), pb = (z, z', w1, w1'), pc = (lo x, lo
+// x', lo y, lo y'), pd = (lo z, lo z', w2, w2') and pg = (g, g', h, h'), where w1 / w2 carry what
+// the pass needs (pass 1 and 3: s*rho and rho; pass 2: charge and effective radius), g the
+// reciprocal effective radius and h the Lennard-Jones code bits (pass 2) or the chain-rule dE/dR
+// (pass 3). prm holds the static per-atom values.
 #ifndef STORMM_B200_UNIT_EVAL_CUH
 #define STORMM_B200_UNIT_EVAL_CUH
 
@@ -492,8 +492,8 @@ __host__ __device__ inline int unitSystems(int max_slots) {
   return n < kMaxUnitSystems ? n : kMaxUnitSystems;
 }
 
-// Dynamic shared memory of one work unit's evaluation by a block of `threads`: max_slots atom slots,
-// max_lj table entries
+// Dynamic shared memory of one work unit's evaluation by a block of `threads`: max_slots atom
+// slots, max_lj table entries
 __host__ __device__ inline size_t unitSmemBytes(int max_slots, int max_lj, int threads) {
   const int max_sys = unitSystems(max_slots);
   size_t b = static_cast<size_t>(kSlotBytes) * max_slots;
@@ -1036,9 +1036,9 @@ __device__ __forceinline__ float2 diagonalWeights(const TileWalk &w, int lane, i
   return f2(1.0f, 1.0f);
 }
 
-// Run one tile: p.pair<false, .>(record, q, 1) for every step, or p.pair<true, .>(record, q, weights)
-// where pairs of weight 0 are to be left out, and p.rotate(source lane) after it.  Padding slots
-// hold parameters that make every contribution to a real atom exactly zero (no charge, zero
+// Run one tile: p.pair<false, .>(record, q, 1) for every step, or p.pair<true, .>(record, q,
+// weights) where pairs of weight 0 are to be left out, and p.rotate(source lane) after it. Padding
+// slots hold parameters that make every contribution to a real atom exactly zero (no charge, zero
 // screened radius and dE/dR, masked Lennard-Jones, far-away coordinates), so partial tiles run the
 // same branch-free loop.
 //
@@ -1048,7 +1048,6 @@ __device__ __forceinline__ float2 diagonalWeights(const TileWalk &w, int lane, i
 template <class P>
 __device__ __forceinline__ void tileFlush(P &) {}
 
-//
 // PLAIN (off-diagonal tiles of the tiled path): no pair of the tile is masked or closer than the
 // distances of tilePlain(), so the passes leave out what only near pairs need.
 template <bool PLAIN = false, class P>
@@ -1386,7 +1385,10 @@ struct PairPass {
       // recovered rounding errors (splitCoordinate): without it the Lennard-Jones energy of a
       // molecule with close contacts errs by up to 1.5e-6 of the root-sum-square of its pair
       // terms.  r2 >= 256 on padding slots, never zero.  Beyond the distance of a plain tile the
-      // Lennard-Jones term is below 1e-5 of a contact's and takes the square of 1/r.
+      // Lennard-Jones term is below 1e-5 of a contact's and takes the square of 1/r: over 30 chains
+      // of 2,500 atoms and four batches of 32 chains the errors against the FP64 mode are the same
+      // to three digits either way (forces of the pair terms 2.5e-7 and 2.8e-7, Lennard-Jones
+      // energy 7.8e-8 and 6.0e-8), and 32 chains take 1,304 us instead of 1,359.
       float2 invr = f2(rsqrtf(r2.x), rsqrtf(r2.y));
       invr = mul2(invr, fma2(mul2(mul2(r2, f2(-0.5f)), invr), invr, f2(1.5f)));
       float2 invr2;
